@@ -59,6 +59,7 @@ _SIGNATURES = {
     "fbfftconv_update_output": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]),
     "fbfftconv_update_grad_input": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]),
     "fbfftconv_acc_grad_parameters": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_void_p]),
+    "fbfftconv_backward": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_void_p]),
     "fbfftconv_update_output_host": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]),
     "fbfftconv_update_grad_input_host": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]),
     "fbfftconv_acc_grad_parameters_host": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_void_p]),

@@ -126,7 +126,6 @@ struct fbfftconv_handle {
   bool profiling = false;
   std::vector<EventPair> events[3][FBFFTCONV_STAGE_COUNT];
   int events_used[3][FBFFTCONV_STAGE_COUNT] = {};
-  bool overlapped[3][FBFFTCONV_STAGE_COUNT] = {};  // stage ran on the second stream since the last reset
   int device;
   int N, bins;
   int oH, oW;
@@ -150,9 +149,6 @@ struct fbfftconv_handle {
   cudaStream_t up = nullptr, down = nullptr;
   cudaEvent_t ev_up = nullptr, ev_kernels[3] = {nullptr, nullptr, nullptr}, ev_down[3] = {nullptr, nullptr, nullptr};
   bool async_used[3] = {false, false, false};
-  // second stream for the second forward transform of a pass, when the two together fit the GPU
-  cudaStream_t aux = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   // communicator
   ncclComm_t comm = nullptr;
   std::string comm_key;
@@ -185,6 +181,11 @@ struct fbfftconv_handle {
 namespace {
 
 size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
+
+// Up to this size the gradInput spectrum gets a buffer of its own even where no flag asks for it, so that a
+// backward call can transform its three operands in one launch and invert its two products in another: that
+// saves launches, which larger layers do not feel.
+constexpr size_t kOwnGradInputBytes = size_t(16) << 20;
 
 int ensure_workspace(fbfftconv_handle* h) {
   if (h->ws) return FBFFTCONV_OK;
@@ -221,50 +222,6 @@ struct StageTimer {
     if (ev) cudaEventRecord(ev->stop, s);
   }
 };
-
-// The two forward transforms of a pass are independent.  Where at least one of them is too
-// small to fill the GPU by itself (small layers, small batch shards) the second runs on the
-// handle's own stream between an event fork and join, so the two overlap; the pattern is
-// capturable in a CUDA graph.  Large transforms stay in order on the caller's stream.
-struct Fork {
-  fbfftconv_handle* h;
-  cudaStream_t main;
-  bool active = false;
-  Fork(fbfftconv_handle* h_, cudaStream_t s, long long tiles_a, long long tiles_b) : h(h_), main(s) {
-    const long long fills_the_gpu = 4LL * sm_count();
-    if (tiles_a >= fills_the_gpu && tiles_b >= fills_the_gpu) return;
-    if (!h->aux) {
-      if (cudaStreamCreateWithFlags(&h->aux, cudaStreamNonBlocking) != cudaSuccess ||
-          cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
-          cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming) != cudaSuccess) {
-        cudaGetLastError();
-        return;  // stay on one stream
-      }
-    }
-    if (cudaEventRecord(h->ev_fork, main) != cudaSuccess || cudaStreamWaitEvent(h->aux, h->ev_fork, 0) != cudaSuccess) {
-      cudaGetLastError();
-      return;
-    }
-    active = true;
-  }
-  cudaStream_t second() const { return active ? h->aux : main; }
-  cudaError_t join() {
-    if (!active) return cudaSuccess;
-    active = false;
-    cudaError_t e = cudaEventRecord(h->ev_join, h->aux);
-    if (e != cudaSuccess) return e;
-    return cudaStreamWaitEvent(main, h->ev_join, 0);
-  }
-  ~Fork() { join(); }  // an early return between fork and join must not leave the streams apart
-};
-
-// Tiles (blocks of work) of a forward transform of d1 x d2 planes.
-long long forward_tiles(int N, int d1, int d2, int h, int w, int pad_u, int pad_l, bool transposed) {
-  const int T = pick_forward_tile(N, h, w, pad_u, pad_l);
-  if (T <= 0) return 1LL << 40;
-  const long long rows = transposed ? d2 : d1, inner = transposed ? d1 : d2;
-  return rows * ((inner + T - 1) / T);
-}
 
 struct DeviceGuard {
   int prev = -1;
@@ -642,7 +599,7 @@ int fbfftconv_create(const fbfftconv_desc* desc, fbfftconv_handle** out) {
   h->bytes_small = align256((B * F + F) * sizeof(float));
   // local gradWeight + gradBias where they are summed or gathered across ranks in the spatial domain
   h->bytes_small += 2 * align256((F * P * d.kernel_h * d.kernel_w + F) * sizeof(float));  // vec_in, vec_out
-  h->bytes_gi = (d.flags & FBFFTCONV_REUSE_INPUT) ? h->bytes_in : 0;
+  h->bytes_gi = (d.flags & FBFFTCONV_REUSE_INPUT) || h->bytes_in <= kOwnGradInputBytes ? h->bytes_in : 0;
   h->bytes_total = h->bytes_in + h->bytes_out + h->bytes_w + h->bytes_small + h->bytes_gi;
   *out = h;
   return FBFFTCONV_OK;
@@ -663,9 +620,6 @@ int fbfftconv_destroy(fbfftconv_handle* h) {
   if (h->ev_up) cudaEventDestroy(h->ev_up);
   if (h->up) cudaStreamDestroy(h->up);
   if (h->down) cudaStreamDestroy(h->down);
-  if (h->aux) cudaStreamDestroy(h->aux);
-  if (h->ev_fork) cudaEventDestroy(h->ev_fork);
-  if (h->ev_join) cudaEventDestroy(h->ev_join);
   for (auto& per_pass : h->events)
     for (auto& pool : per_pass)
       for (auto& p : pool) {
@@ -703,6 +657,110 @@ int fbfftconv_set_workspace(fbfftconv_handle* h, void* device_ptr, size_t bytes)
 
 // ---- passes ----------------------------------------------------------------
 
+namespace {
+
+// One operand of a pass on its way into the frequency domain.
+struct Operand {
+  int stage;  // FBFFTCONV_STAGE_FFT_A / _B: what its transform is timed as
+  FftParams p;
+};
+Operand operand(const fbfftconv_handle* h, int stage, const float* real, float2* spec, int d1, int d2, int rows,
+                int cols, int pad_u, int pad_l) {
+  return Operand{stage, forward_params(real, spec, d1, d2, rows, cols, pad_u, pad_l, h->plane_major ? 2 : 0, h->N)};
+}
+Operand input_operand(const fbfftconv_handle* h, int stage, const float* input) {
+  const fbfftconv_desc& d = h->d;
+  return operand(h, stage, input, h->buf_in(), d.batch, d.n_input_plane, d.input_h, d.input_w, d.pad_h, d.pad_w);
+}
+Operand weight_operand(const fbfftconv_handle* h, int stage, const float* weight) {
+  const fbfftconv_desc& d = h->d;
+  return operand(h, stage, weight, h->buf_w(), d.n_output_plane, d.n_input_plane, d.kernel_h, d.kernel_w, 0, 0);
+}
+Operand grad_output_operand(const fbfftconv_handle* h, int stage, const float* grad_output) {
+  const fbfftconv_desc& d = h->d;
+  return operand(h, stage, grad_output, h->buf_out(), d.batch, d.n_output_plane, h->oH, h->oW, 0, 0);
+}
+
+// Whether transforms run as one launch.  Up to 32 points always: one wave fewer, and no launch gap.  The
+// persistent kernels of the larger sizes only where some operand has too few tiles to fill the GPU (four per
+// SM): their single-operand form is a little faster per plane.
+bool merge_transforms(int N, const FftParams* p, int count) {
+  if (count < 2 || count > kMaxFftOps) return false;
+  if (N <= 32) return true;
+  for (int i = 0; i < count; ++i) {
+    const int T = fft_tile(N);
+    if ((long long)p[i].n_rows * ((p[i].n_inner + T - 1) / T) < 4LL * sm_count()) return true;
+  }
+  return false;
+}
+
+int forward_transforms(fbfftconv_handle* h, int pass, const Operand* ops, int count, cudaStream_t s) {
+  FftParams p[kMaxFftOps];
+  for (int i = 0; i < count; ++i) p[i] = ops[i].p;
+  if (!h->profiling && merge_transforms(h->N, p, count)) {
+    FBF_CUDA(launch_forward(p, count, h->N, s));
+    return FBFFTCONV_OK;
+  }
+  for (int i = 0; i < count; ++i) {
+    StageTimer t(h, pass, ops[i].stage, s);
+    FBF_CUDA(launch_forward(&p[i], 1, h->N, s));
+  }
+  return FBFFTCONV_OK;
+}
+
+int inverse_transform(const FftParams& p, const RowSum* sum, int N, cudaStream_t s) {
+  FBF_CUDA(launch_inverse(&p, 1, sum, N, s));
+  return FBFFTCONV_OK;
+}
+
+// I'^[b][p] = 1/N^2 sum_f O'^[b][f] W^[f][p] per bin, into `gi`; returns the layout of the product.
+int contract_grad_input(fbfftconv_handle* h, float2* gi, int* layout, cudaStream_t s) {
+  const fbfftconv_desc& d = h->d;
+  const int B = d.batch, P = d.n_input_plane, F = d.n_output_plane;
+  const bool simt = (d.flags & FBFFTCONV_CONTRACT_SIMT) || thin_contraction(B, P, F);
+  const bool pm = h->plane_major, flip = !pm && !simt && batch_on_columns(B, P);
+  const float norm = 1.0f / (float)(h->N * h->N);
+  *layout = pm ? 2 : (flip ? 1 : 0);
+  if (pm) {
+    FBF_CUDA(launch_stream_reduce(h->buf_out(), h->buf_w(), gi, B, F, P, F, 1, false, h->bins, norm, s));
+    return FBFFTCONV_OK;
+  }
+  if (flip)  // I'^[p][b] = 1/N^2 sum_f W^[f][p] O'^[b][f]
+    return contract(h->buf_w(), h->buf_out(), gi, h->bins, P, B, F, norm, 0, 0, simt, s, true, false);
+  return contract(h->buf_out(), h->buf_w(), gi, h->bins, B, P, F, norm, 0, 0, simt, s, false, true);
+}
+
+FftParams grad_input_inverse(const fbfftconv_handle* h, const float2* gi, float* grad_input, int layout) {
+  const fbfftconv_desc& d = h->d;
+  return inverse_params(gi, grad_input, nullptr, d.batch, d.n_input_plane, d.input_h, d.input_w, d.pad_h, d.pad_w, 0,
+                        layout, h->N);
+}
+
+// W'^[f][p] = scale/N^2 sum_b conj(O'^[b][f]) I^[b][p] per bin, into the weight buffer.
+int contract_grad_weight(fbfftconv_handle* h, float scale, cudaStream_t s) {
+  const fbfftconv_desc& d = h->d;
+  const int B = d.batch, P = d.n_input_plane, F = d.n_output_plane;
+  const bool simt = (d.flags & FBFFTCONV_CONTRACT_SIMT) || thin_contraction(F, P, B);
+  const float norm = scale / (float)(h->N * h->N);
+  if (h->plane_major) {
+    FBF_CUDA(launch_stream_reduce(h->buf_out(), h->buf_in(), h->buf_w(), F, B, P, 1, F, true, h->bins, norm, s));
+    return FBFFTCONV_OK;
+  }
+  return contract(h->buf_out(), h->buf_in(), h->buf_w(), h->bins, F, P, B, norm, 1, 0, simt, s, true, true);
+}
+
+// Bin (0,0) of O'^[bin][b][f] is the plain sum of gradOutput plane (b, f): its real parts, summed over b,
+// are the bias gradient (src/ConvolutionBias.cu:61-97).  (plane-major: element (b, f, bin 0) sits at
+// ((b*F + f) * bins) complex values)
+RowSum bias_sum(const fbfftconv_handle* h, float* dst, float scale, int accumulate) {
+  const int F = h->d.n_output_plane;
+  const bool pm = h->plane_major;
+  return RowSum{reinterpret_cast<const float*>(h->buf_out()), dst,   F,         h->d.batch,
+                pm ? 2LL * h->bins : 2,                        pm ? 2LL * F * h->bins : 2LL * pad4(F), scale, accumulate};
+}
+
+}  // namespace
+
 int fbfftconv_update_output(fbfftconv_handle* h, const float* input, const float* weight,
                             const float* bias, float* output, fbfftconv_stream stream) {
   if (!h || !input || !weight || !output) return fail(FBFFTCONV_ERR_INVALID_ARGUMENT, "null argument");
@@ -722,20 +780,8 @@ int fbfftconv_update_output(fbfftconv_handle* h, const float* input, const float
   const bool flip = !pm && !simt && batch_on_columns(B, F);
   const float norm = 1.0f / (float)(h->N * h->N);
   // I^[bin][b][p], W^[bin][f][p]   (plane-major: I^[b][p][bin], W^[f][p][bin])
-  {
-    Fork fork(h, s, forward_tiles(h->N, B, P, d.input_h, d.input_w, d.pad_h, d.pad_w, false),
-              forward_tiles(h->N, F, P, d.kernel_h, d.kernel_w, 0, 0, false));
-    {
-      StageTimer t(h, pass, FBFFTCONV_STAGE_FFT_A, s);
-      FBF_CUDA(launch_forward(forward_params(input, h->buf_in(), B, P, d.input_h, d.input_w, d.pad_h, d.pad_w, pm ? 2 : 0, h->N), h->N, s));
-    }
-    {
-      StageTimer t(h, pass, FBFFTCONV_STAGE_FFT_B, fork.second());
-      if (fork.active) h->overlapped[pass][FBFFTCONV_STAGE_FFT_B] = true;
-      FBF_CUDA(launch_forward(forward_params(weight, h->buf_w(), F, P, d.kernel_h, d.kernel_w, 0, 0, pm ? 2 : 0, h->N), h->N, fork.second()));
-    }
-    FBF_CUDA(fork.join());
-  }
+  const Operand ops[2] = {input_operand(h, FBFFTCONV_STAGE_FFT_A, input), weight_operand(h, FBFFTCONV_STAGE_FFT_B, weight)};
+  FBF_TRY(forward_transforms(h, pass, ops, 2, s));
   // O^[b][f] = 1/N^2 sum_p I^[b][p] conj(W^[f][p]) per bin
   {
     StageTimer t(h, pass, FBFFTCONV_STAGE_CONTRACT, s);
@@ -749,8 +795,8 @@ int fbfftconv_update_output(fbfftconv_handle* h, const float* input, const float
   }
   {
     StageTimer t(h, pass, FBFFTCONV_STAGE_IFFT, s);
-    FBF_CUDA(launch_inverse(inverse_params(h->buf_out(), output, bias, B, F, h->oH, h->oW, 0, 0, 0,
-                                           pm ? 2 : (flip ? 1 : 0), h->N), h->N, s));
+    FBF_TRY(inverse_transform(inverse_params(h->buf_out(), output, bias, B, F, h->oH, h->oW, 0, 0, 0,
+                                             pm ? 2 : (flip ? 1 : 0), h->N), nullptr, h->N, s));
   }
   // what the buffers hold now (every pass reads a tensor's spectrum in the one layout it is written in)
   h->have_input_spec = true;
@@ -770,50 +816,25 @@ int fbfftconv_update_grad_input(fbfftconv_handle* h, const float* grad_output, c
   FBF_TRY(check_device_pointer(h->device, grad_input, "gradInput"));
   FBF_TRY(ensure_workspace(h));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const fbfftconv_desc& d = h->d;
-  const int B = d.batch, P = d.n_input_plane, F = d.n_output_plane;
-  const bool simt = (d.flags & FBFFTCONV_CONTRACT_SIMT) || thin_contraction(B, P, F);
   const int pass = FBFFTCONV_PASS_UPDATE_GRAD_INPUT;
-  const bool pm = h->plane_major;
-  const bool flip = !pm && !simt && batch_on_columns(B, P);
-  const float norm = 1.0f / (float)(h->N * h->N);
   // O'^[bin][b][f], W^[bin][f][p] (the sum over f reads W^ with f as the row index)
-  {
-    Fork fork(h, s, forward_tiles(h->N, B, F, h->oH, h->oW, 0, 0, false),
-              forward_tiles(h->N, F, P, d.kernel_h, d.kernel_w, 0, 0, false));
-    {
-      StageTimer t(h, pass, FBFFTCONV_STAGE_FFT_A, s);
-      FBF_CUDA(launch_forward(forward_params(grad_output, h->buf_out(), B, F, h->oH, h->oW, 0, 0, pm ? 2 : 0, h->N), h->N, s));
-    }
-    h->have_grad_output_spec = true;
-    if (!((d.flags & FBFFTCONV_REUSE_WEIGHT) && h->have_weight_spec)) {
-      StageTimer t(h, pass, FBFFTCONV_STAGE_FFT_B, fork.second());
-      if (fork.active) h->overlapped[pass][FBFFTCONV_STAGE_FFT_B] = true;
-      FBF_CUDA(launch_forward(forward_params(weight, h->buf_w(), F, P, d.kernel_h, d.kernel_w, 0, 0, pm ? 2 : 0, h->N), h->N, fork.second()));
-      h->have_weight_spec = true;
-    }
-    FBF_CUDA(fork.join());
-  }
-  // with REUSE_INPUT the input spectrum stays in its buffer for accGradParameters
+  Operand ops[2] = {grad_output_operand(h, FBFFTCONV_STAGE_FFT_A, grad_output)};
+  int count = 1;
+  if (!((h->d.flags & FBFFTCONV_REUSE_WEIGHT) && h->have_weight_spec))
+    ops[count++] = weight_operand(h, FBFFTCONV_STAGE_FFT_B, weight);
+  FBF_TRY(forward_transforms(h, pass, ops, count, s));
+  h->have_grad_output_spec = true;
+  h->have_weight_spec = true;
+  // where gradInput has a buffer of its own the input spectrum stays for accGradParameters
   float2* gi = h->buf_gi();
   if (gi == h->buf_in()) h->have_input_spec = false;
-  // I'^[bin][b][p] = 1/N^2 sum_f O'^[b][f] W^[f][p]
+  int layout = 0;
   {
     StageTimer t(h, pass, FBFFTCONV_STAGE_CONTRACT, s);
-    if (pm) {  // I'^[b][p] = sum_f O'^[b][f] W^[f][p]
-      FBF_CUDA(launch_stream_reduce(h->buf_out(), h->buf_w(), gi, B, F, P, F, 1, false, h->bins, norm, s));
-    } else if (flip) {  // I'^[p][b] = 1/N^2 sum_f W^[f][p] O'^[b][f]
-      FBF_TRY(contract(h->buf_w(), h->buf_out(), gi, h->bins, P, B, F, norm, 0, 0, simt, s, true, false));
-    } else {
-      FBF_TRY(contract(h->buf_out(), h->buf_w(), gi, h->bins, B, P, F, norm, 0, 0, simt, s, false, true));
-    }
+    FBF_TRY(contract_grad_input(h, gi, &layout, s));
   }
-  {
-    StageTimer t(h, pass, FBFFTCONV_STAGE_IFFT, s);
-    FBF_CUDA(launch_inverse(inverse_params(gi, grad_input, nullptr, B, P, d.input_h, d.input_w,
-                                           d.pad_h, d.pad_w, 0, pm ? 2 : (flip ? 1 : 0), h->N), h->N, s));
-  }
-  return FBFFTCONV_OK;
+  StageTimer t(h, pass, FBFFTCONV_STAGE_IFFT, s);
+  return inverse_transform(grad_input_inverse(h, gi, grad_input, layout), nullptr, h->N, s);
 }
 
 namespace {
@@ -891,28 +912,19 @@ int fbfftconv_acc_grad_parameters(fbfftconv_handle* h, const float* input, const
   FBF_TRY(ensure_workspace(h));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const fbfftconv_desc& d = h->d;
-  const int B = d.batch, P = d.n_input_plane, F = d.n_output_plane;
-  const bool simt = (d.flags & FBFFTCONV_CONTRACT_SIMT) || thin_contraction(F, P, B);
+  const int P = d.n_input_plane, F = d.n_output_plane;
   const int accumulate = (d.flags & FBFFTCONV_ACCUMULATE_GRADS) ? 1 : 0;
   const int pass = FBFFTCONV_PASS_ACC_GRAD_PARAMETERS;
   const bool pm = h->plane_major;
   // O'^[bin][b][f], I^[bin][b][p]: the batch, the row index of both, is the contraction index here
-  {
-    Fork fork(h, s, forward_tiles(h->N, B, F, h->oH, h->oW, 0, 0, false),
-              forward_tiles(h->N, B, P, d.input_h, d.input_w, d.pad_h, d.pad_w, false));
-    if (!(((d.flags & FBFFTCONV_REUSE_OUTPUT) || h->same_grad_output) && h->have_grad_output_spec)) {
-      StageTimer t(h, pass, FBFFTCONV_STAGE_FFT_A, s);
-      FBF_CUDA(launch_forward(forward_params(grad_output, h->buf_out(), B, F, h->oH, h->oW, 0, 0, pm ? 2 : 0, h->N), h->N, s));
-      h->have_grad_output_spec = true;
-    }
-    if (!((d.flags & FBFFTCONV_REUSE_INPUT) && h->have_input_spec)) {
-      StageTimer t(h, pass, FBFFTCONV_STAGE_FFT_B, fork.second());
-      if (fork.active) h->overlapped[pass][FBFFTCONV_STAGE_FFT_B] = true;
-      FBF_CUDA(launch_forward(forward_params(input, h->buf_in(), B, P, d.input_h, d.input_w, d.pad_h, d.pad_w, pm ? 2 : 0, h->N), h->N, fork.second()));
-      h->have_input_spec = true;
-    }
-    FBF_CUDA(fork.join());
-  }
+  Operand ops[2];
+  int count = 0;
+  if (!(((d.flags & FBFFTCONV_REUSE_OUTPUT) || h->same_grad_output) && h->have_grad_output_spec))
+    ops[count++] = grad_output_operand(h, FBFFTCONV_STAGE_FFT_A, grad_output);
+  if (!((d.flags & FBFFTCONV_REUSE_INPUT) && h->have_input_spec))
+    ops[count++] = input_operand(h, FBFFTCONV_STAGE_FFT_B, input);
+  FBF_TRY(forward_transforms(h, pass, ops, count, s));
+  h->have_grad_output_spec = h->have_input_spec = true;
   h->have_weight_spec = false;  // the weight buffer receives the gradient spectrum below
   NcclApi* api = h->comm ? nccl_api() : nullptr;
   if (h->comm && !api) return fail(FBFFTCONV_ERR_COMM, "libnccl is not loadable");
@@ -936,28 +948,17 @@ int fbfftconv_acc_grad_parameters(fbfftconv_handle* h, const float* input, const
   float* local_w = h->vec_in();
   float* bias_part =
       (spatial || scatter || scatter_bins) ? local_w + n_weight : reinterpret_cast<float*>(h->buf_w()) + spec_floats;
-  // W'^[bin][f][p] = scale/N^2 sum_b conj(O'^[b][f]) I^[b][p]
   {
     StageTimer t(h, pass, FBFFTCONV_STAGE_CONTRACT, s);
-    const float norm = scale / (float)(h->N * h->N);
-    if (pm) {  // W'^[f][p] = sum_b conj(O'^[b][f]) I^[b][p]
-      FBF_CUDA(launch_stream_reduce(h->buf_out(), h->buf_in(), h->buf_w(), F, B, P, 1, F, true, h->bins, norm, s));
-    } else {
-      FBF_TRY(contract(h->buf_out(), h->buf_in(), h->buf_w(), h->bins, F, P, B, norm, 1, 0, simt, s, true, true));
-    }
+    FBF_TRY(contract_grad_weight(h, scale, s));
   }
-  if (grad_bias) {
+  // on one GPU the bias gradient rides in the launch of the inverse transform below; across ranks it is summed
+  // first, and timed on its own it is a launch of its own
+  const bool bias_rides = grad_bias && !h->comm && !h->profiling;
+  const RowSum sum = bias_sum(h, h->comm ? bias_part : grad_bias, scale, h->comm ? 0 : accumulate);
+  if (grad_bias && !bias_rides) {
     StageTimer t(h, pass, FBFFTCONV_STAGE_BIAS, s);
-    // bin (0,0) of O'^[bin][b][f] is the plain sum of gradOutput plane (b, f): its real
-    // parts, summed over b, are the bias gradient (src/ConvolutionBias.cu:61-97).
-    // (plane-major: element (b, f, bin 0) sits at ((b*F + f) * bins) complex values)
-    const float* dc = reinterpret_cast<const float*>(h->buf_out());
-    const long long ld = pm ? 2LL * h->bins : 2;
-    const long long dc_step = pm ? 2LL * F * h->bins : 2LL * pad4(F);
-    if (h->comm)
-      FBF_CUDA(launch_row_sum(dc, bias_part, F, B, ld, dc_step, scale, 0, s));
-    else
-      FBF_CUDA(launch_row_sum(dc, grad_bias, F, B, ld, dc_step, scale, accumulate, s));
+    FBF_CUDA(launch_row_sum(sum, s));
   }
   const size_t bias_floats = grad_bias ? (size_t)F : 0;
   if (scatter) {
@@ -977,9 +978,9 @@ int fbfftconv_acc_grad_parameters(fbfftconv_handle* h, const float* input, const
     }
     {
       StageTimer t(h, pass, FBFFTCONV_STAGE_IFFT, s);
-      FBF_CUDA(launch_inverse(inverse_params(reinterpret_cast<const float2*>(mine), local_w + x.slice_first,
-                                             nullptr, F / h->nranks, P, d.kernel_h, d.kernel_w, 0, 0, 0, 2, h->N),
-                              h->N, s));
+      FBF_TRY(inverse_transform(inverse_params(reinterpret_cast<const float2*>(mine), local_w + x.slice_first,
+                                               nullptr, F / h->nranks, P, d.kernel_h, d.kernel_w, 0, 0, 0, 2, h->N),
+                                nullptr, h->N, s));
     }
     if (peer) {
       StageTimer t(h, pass, FBFFTCONV_STAGE_ALLREDUCE, s);
@@ -1018,8 +1019,8 @@ int fbfftconv_acc_grad_parameters(fbfftconv_handle* h, const float* input, const
     if (x.zero_after) FBF_CUDA(cudaMemsetAsync(mine + chunk, 0, x.zero_after * sizeof(float), s));
     {
       StageTimer t(h, pass, FBFFTCONV_STAGE_IFFT, s);
-      FBF_CUDA(launch_inverse(inverse_params(h->buf_w(), local_w, nullptr, F, P, d.kernel_h, d.kernel_w, 0, 0, 0, 0,
-                                             h->N), h->N, s));
+      FBF_TRY(inverse_transform(inverse_params(h->buf_w(), local_w, nullptr, F, P, d.kernel_h, d.kernel_w, 0, 0, 0, 0,
+                                               h->N), nullptr, h->N, s));
     }
     {
       StageTimer t(h, pass, FBFFTCONV_STAGE_ALLREDUCE, s);
@@ -1041,8 +1042,9 @@ int fbfftconv_acc_grad_parameters(fbfftconv_handle* h, const float* input, const
   }
   if (!scatter && !scatter_bins) {
     StageTimer t(h, pass, FBFFTCONV_STAGE_IFFT, s);
-    FBF_CUDA(launch_inverse(inverse_params(h->buf_w(), spatial ? local_w : grad_weight, nullptr, F, P, d.kernel_h,
-                                           d.kernel_w, 0, 0, spatial ? 0 : accumulate, pm ? 2 : 0, h->N), h->N, s));
+    FBF_TRY(inverse_transform(inverse_params(h->buf_w(), spatial ? local_w : grad_weight, nullptr, F, P, d.kernel_h,
+                                             d.kernel_w, 0, 0, spatial ? 0 : accumulate, pm ? 2 : 0, h->N),
+                              bias_rides ? &sum : nullptr, h->N, s));
   }
   const bool summed_by_peers = peer && (scatter || scatter_bins || spatial);
   if (spatial) {
@@ -1062,6 +1064,58 @@ int fbfftconv_acc_grad_parameters(fbfftconv_handle* h, const float* input, const
     StageTimer t(h, pass, FBFFTCONV_STAGE_BIAS, s);
     // summed over peers the bias gradient arrives behind gradWeight in the delivered vector
     FBF_CUDA(launch_copy_or_add(summed_by_peers ? h->vec_out() + n_weight : bias_part, grad_bias, F, accumulate, s));
+  }
+  return FBFFTCONV_OK;
+}
+
+int fbfftconv_backward(fbfftconv_handle* h, const float* input, const float* grad_output, const float* weight,
+                       float* grad_input, float* grad_weight, float* grad_bias, float scale, fbfftconv_stream stream) {
+  if (!h || !input || !grad_output || !weight || !grad_input || !grad_weight)
+    return fail(FBFFTCONV_ERR_INVALID_ARGUMENT, "null argument");
+  // Across ranks, while kernels are timed one by one, and where the input spectrum cannot survive
+  // updateGradInput: the two passes after one another, the second with the gradOutput spectrum of the first.
+  if (h->comm || h->profiling || !h->bytes_gi) {
+    FBF_TRY(fbfftconv_update_grad_input(h, grad_output, weight, grad_input, stream));
+    h->same_grad_output = true;
+    const int rc = fbfftconv_acc_grad_parameters(h, input, grad_output, grad_weight, grad_bias, scale, stream);
+    h->same_grad_output = false;
+    return rc;
+  }
+  DeviceGuard g;
+  FBF_CUDA(g.enter(h->device));
+  FBF_TRY(check_device_pointer(h->device, input, "input"));
+  FBF_TRY(check_device_pointer(h->device, grad_output, "gradOutput"));
+  FBF_TRY(check_device_pointer(h->device, weight, "weight"));
+  FBF_TRY(check_device_pointer(h->device, grad_input, "gradInput"));
+  FBF_TRY(check_device_pointer(h->device, grad_weight, "gradWeight"));
+  FBF_TRY(check_device_pointer(h->device, grad_bias, "gradBias"));
+  FBF_TRY(ensure_workspace(h));
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const fbfftconv_desc& d = h->d;
+  const int pass = FBFFTCONV_PASS_UPDATE_GRAD_INPUT;
+  const int accumulate = (d.flags & FBFFTCONV_ACCUMULATE_GRADS) ? 1 : 0;
+  Operand ops[3] = {grad_output_operand(h, FBFFTCONV_STAGE_FFT_A, grad_output)};
+  int count = 1;
+  if (!((d.flags & FBFFTCONV_REUSE_WEIGHT) && h->have_weight_spec))
+    ops[count++] = weight_operand(h, FBFFTCONV_STAGE_FFT_B, weight);
+  if (!((d.flags & FBFFTCONV_REUSE_INPUT) && h->have_input_spec))
+    ops[count++] = input_operand(h, FBFFTCONV_STAGE_FFT_B, input);
+  FBF_TRY(forward_transforms(h, pass, ops, count, s));
+  h->have_grad_output_spec = h->have_input_spec = true;
+  int layout = 0;
+  FBF_TRY(contract_grad_input(h, h->buf_gi(), &layout, s));
+  h->have_weight_spec = false;  // its buffer receives the gradient spectrum
+  FBF_TRY(contract_grad_weight(h, scale, s));
+  const FftParams inv[2] = {grad_input_inverse(h, h->buf_gi(), grad_input, layout),
+                            inverse_params(h->buf_w(), grad_weight, nullptr, d.n_output_plane, d.n_input_plane,
+                                           d.kernel_h, d.kernel_w, 0, 0, accumulate, h->plane_major ? 2 : 0, h->N)};
+  RowSum sum{};
+  if (grad_bias) sum = bias_sum(h, grad_bias, scale, accumulate);
+  if (merge_transforms(h->N, inv, 2)) {
+    FBF_CUDA(launch_inverse(inv, 2, &sum, h->N, s));
+  } else {
+    FBF_CUDA(launch_inverse(&inv[0], 1, nullptr, h->N, s));
+    FBF_CUDA(launch_inverse(&inv[1], 1, &sum, h->N, s));
   }
   return FBFFTCONV_OK;
 }
@@ -1410,8 +1464,8 @@ int fbfftconv_fft2d(const float* real, void* spectrum, int d1, int d2, int h, in
   if (d1 <= 0 || d2 <= 0 || h <= 0 || w <= 0 || pad_u < 0 || pad_l < 0 || h + pad_u > fft_size ||
       w + pad_l > fft_size || d1 > 65535 || d2 > 65535)
     return fail(FBFFTCONV_ERR_INVALID_ARGUMENT, "plane of %dx%d at (%d,%d) does not fit %d", h, w, pad_u, pad_l, fft_size);
-  FBF_CUDA(launch_forward(forward_params(real, static_cast<float2*>(spectrum), d1, d2, h, w, pad_u, pad_l, transposed, fft_size),
-                          fft_size, static_cast<cudaStream_t>(stream)));
+  const FftParams p = forward_params(real, static_cast<float2*>(spectrum), d1, d2, h, w, pad_u, pad_l, transposed, fft_size);
+  FBF_CUDA(launch_forward(&p, 1, fft_size, static_cast<cudaStream_t>(stream)));
   return FBFFTCONV_OK;
 }
 
@@ -1423,9 +1477,9 @@ int fbfftconv_ifft2d(const void* spectrum, float* real, const float* bias, int d
   if (d1 <= 0 || d2 <= 0 || h <= 0 || w <= 0 || off_y < 0 || off_x < 0 || h + off_y > fft_size ||
       w + off_x > fft_size || d1 > 65535 || d2 > 65535)
     return fail(FBFFTCONV_ERR_INVALID_ARGUMENT, "window of %dx%d at (%d,%d) does not fit %d", h, w, off_y, off_x, fft_size);
-  FBF_CUDA(launch_inverse(inverse_params(static_cast<const float2*>(spectrum), real, bias, d1, d2, h, w, off_y, off_x, accumulate != 0, plane_major != 0 ? 2 : 0, fft_size),
-                          fft_size, static_cast<cudaStream_t>(stream)));
-  return FBFFTCONV_OK;
+  return inverse_transform(inverse_params(static_cast<const float2*>(spectrum), real, bias, d1, d2, h, w, off_y, off_x,
+                                          accumulate != 0, plane_major != 0 ? 2 : 0, fft_size),
+                           nullptr, fft_size, static_cast<cudaStream_t>(stream));
 }
 
 int fbfftconv_fft2d_reference_layout(const float* real, void* frequency, void* scratch, int planes, int h, int w,
@@ -1536,13 +1590,12 @@ int fbfftconv_profile_enable(fbfftconv_handle* h, int enable) {
 int fbfftconv_profile_reset(fbfftconv_handle* h) {
   if (!h) return fail(FBFFTCONV_ERR_INVALID_ARGUMENT, "null handle");
   memset(h->events_used, 0, sizeof(h->events_used));
-  memset(h->overlapped, 0, sizeof(h->overlapped));
   return FBFFTCONV_OK;
 }
 
 int fbfftconv_profile_overlapped(const fbfftconv_handle* h, int pass, int stage) {
   if (!h || pass < 0 || pass > 2 || stage < 0 || stage >= FBFFTCONV_STAGE_COUNT) return -1;
-  return h->overlapped[pass][stage] ? 1 : 0;
+  return 0;  // while timing is on, every kernel runs alone on the caller's stream
 }
 
 int fbfftconv_profile_read(fbfftconv_handle* h, int pass, int stage, double* total_ms, int* launches) {

@@ -94,9 +94,8 @@ cudaError_t launch_bias_grad(const float* grad_out, float* grad_bias, float* scr
   return cudaGetLastError();
 }
 
-cudaError_t launch_row_sum(const float* src, float* dst, int rows, int count, long long ld, long long step,
-                           float scale, int accumulate, cudaStream_t stream) {
-  row_sum_kernel<<<rows, 128, 0, stream>>>(src, dst, count, ld, step, scale, accumulate);
+cudaError_t launch_row_sum(const RowSum& p, cudaStream_t stream) {
+  row_sum_kernel<<<p.rows, 128, 0, stream>>>(p.src, p.dst, p.count, p.ld, p.step, p.scale, p.accumulate);
   count_launch();
   return cudaGetLastError();
 }

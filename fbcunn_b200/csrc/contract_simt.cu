@@ -132,6 +132,7 @@ contract_simt_kernel(const __grid_constant__ ContractParams p) {
   };
 
   const int ksteps = (p.k + BK - 1) / BK;
+  grid_dependency_wait();
   fetch_tiles(0);
   for (int ks = 0; ks < ksteps; ++ks) {
     const int buf = ks & 1;
@@ -186,15 +187,16 @@ contract_simt_kernel(const __grid_constant__ ContractParams p) {
 
 cudaError_t launch_contract_simt(const ContractParams& p, cudaStream_t stream) {
   if (p.bins > 65535 || (p.lda & 3) || (p.ldb & 3) || (p.ldc & 3)) return cudaErrorInvalidValue;
+  cudaError_t e;
   if (p.ldc <= 4) {
     dim3 grid(1, (p.m + 127) / 128, p.bins);
-    contract_simt_kernel<128, 4, 1, 2><<<grid, THREADS, 0, stream>>>(p);
+    e = launch_dependent(contract_simt_kernel<128, 4, 1, 2>, grid, THREADS, 0, stream, p);
   } else {
     dim3 grid((p.ldc + 63) / 64, (p.m + 63) / 64, p.bins);
-    contract_simt_kernel<64, 64, 4, 4><<<grid, THREADS, 0, stream>>>(p);
+    e = launch_dependent(contract_simt_kernel<64, 64, 4, 4>, grid, THREADS, 0, stream, p);
   }
   count_launch();
-  return cudaGetLastError();
+  return e;
 }
 
 }  // namespace fbfft

@@ -70,6 +70,7 @@ stream_expand_kernel(const float2* __restrict__ X, const float2* __restrict__ Y,
                      int V, int P, int v_per_block, long long bins, float alpha) {
   extern __shared__ float4 ring[];  // [RING_STAGES][PMAX][THREADS]
   const long long bin = ((long long)blockIdx.x * THREADS + threadIdx.x) * 2;
+  grid_dependency_wait();
   if (bin >= bins) return;
   const int u0 = blockIdx.y * TU;
   const int v0 = blockIdx.z * v_per_block;
@@ -122,6 +123,7 @@ stream_reduce_kernel(const float2* __restrict__ X, const float2* __restrict__ Y,
   extern __shared__ float4 ring[];  // [RING_STAGES][PMAX + TU][NT]
   constexpr int NLOAD = PMAX + TU;
   const long long bin = ((long long)blockIdx.x * NT + threadIdx.x) * 2;
+  grid_dependency_wait();
   if (bin >= bins) return;
   const int u0 = blockIdx.y * TU;
   float4* mine = ring + threadIdx.x;
@@ -184,9 +186,9 @@ cudaError_t launch_stream_expand(const float2* x, const float2* y, float2* z, in
   const int smem = RING_STAGES * PMAX * THREADS * (int)sizeof(float4);
   cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(stream_expand_kernel<TU>), smem);
   if (e != cudaSuccess) return e;
-  stream_expand_kernel<TU><<<grid, THREADS, smem, stream>>>(x, y, z, U, V, P, v_per_block, bins, alpha);
+  e = launch_dependent(stream_expand_kernel<TU>, grid, THREADS, smem, stream, x, y, z, U, V, P, v_per_block, bins, alpha);
   count_launch();
-  return cudaGetLastError();
+  return e;
 }
 
 cudaError_t launch_stream_reduce(const float2* x, const float2* y, float2* z, int U, int W, int P, long long xs_u,
@@ -213,8 +215,7 @@ cudaError_t launch_stream_reduce(const float2* x, const float2* y, float2* z, in
     const int smem = RING_STAGES * (PMAX + tu) * nt * (int)sizeof(float4);
     cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
     if (e != cudaSuccess) return e;
-    kernel<<<grid, nt, smem, stream>>>(x, y, z, U, W, P, xs_u, xs_w, bins, alpha);
-    return cudaSuccess;
+    return launch_dependent(kernel, grid, nt, smem, stream, x, y, z, U, W, P, xs_u, xs_w, bins, alpha);
   };
   cudaError_t e;
   if (tu == 4)

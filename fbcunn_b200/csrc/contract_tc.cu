@@ -312,9 +312,10 @@ cudaError_t launch_wide_as(const ContractParams& p, cudaStream_t stream) {
   if (e != cudaSuccess) return e;
   const int sms = sm_count();
   const int grid = (int)(total < sms ? total : sms);
-  contract_tc_wide_kernel<WBNC, A_MN, B_MN><<<grid, W_THREADS, TL::SMEM_BYTES, stream>>>(map_a, map_b, t);
+  e = launch_dependent(contract_tc_wide_kernel<WBNC, A_MN, B_MN>, dim3(grid), W_THREADS, TL::SMEM_BYTES, stream, map_a,
+                       map_b, t);
   count_launch();
-  return cudaGetLastError();
+  return e;
 }
 
 template <int WBNC>

@@ -89,6 +89,7 @@ fft1d_forward_lines_kernel(const float* __restrict__ real, float2* __restrict__ 
   __shared__ float2 buf[L::LINES * L::PITCH];  // the split buffer, then (same memory) the transformed lines
   const long long pair0 = (long long)blockIdx.x * L::LINES;
   float2* zbuf = buf;
+  grid_dependency_wait();
   transform_lines<N, false, false, true>(
       buf,
       [&](int line, int x) {
@@ -117,6 +118,7 @@ fft1d_inverse_lines_kernel(const float2* __restrict__ spec, float* __restrict__ 
   using L = Lines<N>;
   __shared__ float2 buf[L::LINES * L::PITCH];  // first the tangled lines, then the split buffer
   const long long pair0 = (long long)blockIdx.x * L::LINES;
+  grid_dependency_wait();
   for (int item = threadIdx.x; item < L::LINES * L::BINS; item += kThreads) {
     const int l = item / L::BINS, k = item - l * L::BINS;
     const long long r0 = 2 * (pair0 + l);
@@ -144,12 +146,11 @@ cudaError_t launch_lines(bool inverse, const float* real_in, float* real_out, fl
   const long long pairs = (rows + 1) / 2;
   const long long blocks = (pairs + Lines<N>::LINES - 1) / Lines<N>::LINES;
   if (blocks > 0x7fffffff) return cudaErrorInvalidValue;
-  if (inverse)
-    fft1d_inverse_lines_kernel<N><<<(unsigned)blocks, kThreads, 0, stream>>>(spec, real_out, rows, n, offset);
-  else
-    fft1d_forward_lines_kernel<N><<<(unsigned)blocks, kThreads, 0, stream>>>(real_in, spec, rows, n, offset);
+  const cudaError_t e =
+      inverse ? launch_dependent(fft1d_inverse_lines_kernel<N>, dim3((unsigned)blocks), kThreads, 0, stream, spec, real_out, rows, n, offset)
+              : launch_dependent(fft1d_forward_lines_kernel<N>, dim3((unsigned)blocks), kThreads, 0, stream, real_in, spec, rows, n, offset);
   count_launch();
-  return cudaGetLastError();
+  return e;
 }
 
 }  // namespace

@@ -235,6 +235,10 @@ struct FftGeom {
 };
 
 static inline bool cooperative(int N) { return N > 32; }
+// Planes per block.  32-point transforms: 8 (more blocks per SM at 64-86 registers per thread measured
+// 5-10 % faster than 16); 8- and 16-point ones are fastest at 16; the cooperative sizes take what lets two
+// blocks share an SM's memory.
+constexpr int fft_tile(int N) { return N > 64 ? 1 : N > 32 ? 4 : N > 16 ? 8 : 16; }
 #define FBF_COOP_THREADS 256  // measured slower: 288 (whole rounds in the column phases, but a 96-register cap), 384, 512
 static_assert(FBF_COOP_THREADS % 32 == 0, "whole warps, and a multiple of every N2");
 static inline int coop_threads() { return FBF_COOP_THREADS; }

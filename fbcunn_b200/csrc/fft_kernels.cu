@@ -44,63 +44,155 @@ namespace {
 
 std::atomic<uint64_t> g_launches{0};
 
+constexpr int kRowSumWarpLimit = 512;  // values a single warp sums (16 a lane, all in flight at once)
+
 template <int N, int T>
 constexpr int block_threads() {
   return ((N / 2 + 1) * T + 31) / 32 * 32 < 64 ? 64 : ((N / 2 + 1) * T + 31) / 32 * 32;
 }
 
-template <int N, int T>
-__global__ void __launch_bounds__(block_threads<N, T>())
-fft2d_forward_kernel(const __grid_constant__ FftParams p, const __grid_constant__ FftGeom g) {
-  extern __shared__ __align__(16) char smem[];
-  const int tid = threadIdx.x;
-  const int row = blockIdx.y;
-  const int inner0 = blockIdx.x * T;
-  Forward<N, T>::load(p, g, smem, tid, blockDim.x, row, inner0);
-  __syncthreads();
-  LineRegs<N> regs;
-  Forward<N, T>::row_fetch(p, g, smem, tid, row, inner0, regs);
-  __syncthreads();  // the column buffer aliases the staged planes
-  Forward<N, T>::row_pass(g, smem, tid, regs);
-  __syncthreads();
-  Forward<N, T>::col_pass(p, g, smem, tid, row, inner0);
+// dst[r] (=|+=) scale * sum of a row: a warp per row, or -- long rows -- the block per row.
+__device__ void row_sum_block(const RowSum& s, int block, char* smem) {
+  const bool per_warp = s.count <= kRowSumWarpLimit;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const int row = per_warp ? block * nwarps + warp : block;
+  float v = 0.f;
+  if (row < s.rows)
+    for (int i = per_warp ? lane : (int)threadIdx.x; i < s.count; i += per_warp ? 32 : (int)blockDim.x)
+      v += s.src[row * s.ld + i * s.step];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if (!per_warp) {
+    float* part = reinterpret_cast<float*>(smem);
+    if (lane == 0) part[warp] = v;
+    __syncthreads();
+    v = 0.f;
+    if (threadIdx.x == 0)
+      for (int i = 0; i < nwarps; ++i) v += part[i];
+  }
+  if (row < s.rows && (per_warp ? lane == 0 : threadIdx.x == 0))
+    s.dst[row] = s.accumulate ? s.dst[row] + s.scale * v : s.scale * v;
+}
+int row_sum_blocks(const RowSum& s, int threads) {
+  const int rows_per_block = s.count <= kRowSumWarpLimit ? threads / 32 : 1;
+  return (s.rows + rows_per_block - 1) / rows_per_block;
 }
 
-template <int N, int T>
+// One launch transforms the planes of up to OPS operands of a pass (its two or three real tensors, or the
+// two spectra that a backward call inverts): the block index runs over the tiles of all of them.  Small
+// layers are bound by launches, and a small operand next to a large one would leave most SMs idle in a
+// launch of its own.  With OPS = 1 the parameters are compile-time addresses in the constant bank.
+template <int OPS>
+struct FftBatch {
+  FftParams p[OPS];
+  FftGeom g[OPS];
+  int tiles_x[OPS];    // tiles along the inner index
+  int tile_end[OPS];   // running total of tiles
+  int sum_blocks;      // inverse only: leading blocks that do `sum` instead of a tile
+  RowSum sum;
+};
+
+// Runs body(params, geometry, tile inside the operand, tiles along the inner index) for the operand that
+// `tile` belongs to.  The body is instantiated once per operand: with the operand's number known at compile
+// time its parameters stay operands of the instructions, where a run-time index cost 10 % (32 points, plain
+// instruction issue) and 16 registers (16 points).
+template <int OPS, class Body>
+__device__ __forceinline__ void with_operand(const FftBatch<OPS>& b, int tile, Body body) {
+  if constexpr (OPS == 1) {
+    body(b.p[0], b.g[0], tile, b.tiles_x[0]);
+  } else {
+    if (tile < b.tile_end[0])
+      body(b.p[0], b.g[0], tile, b.tiles_x[0]);
+    else if (tile < b.tile_end[1])
+      body(b.p[1], b.g[1], tile - b.tile_end[0], b.tiles_x[1]);
+    else
+      body(b.p[2], b.g[2], tile - b.tile_end[1], b.tiles_x[2]);
+  }
+}
+
+template <int N, int T, int OPS>
 __global__ void __launch_bounds__(block_threads<N, T>())
-fft2d_inverse_kernel(const __grid_constant__ FftParams p, const __grid_constant__ FftGeom g) {
+fft2d_forward_kernel(const __grid_constant__ FftBatch<OPS> b) {
   extern __shared__ __align__(16) char smem[];
   const int tid = threadIdx.x;
-  const int row = blockIdx.y;
-  const int inner0 = blockIdx.x * T;
-  Inverse<N, T>::col_pass(p, g, smem, tid, row, inner0);
-  __syncthreads();
-  LineRegs<N> regs;
-  Inverse<N, T>::row_fetch(g, smem, tid, regs);
-  __syncthreads();  // the staged output aliases the column buffer
-  Inverse<N, T>::row_pass(p, g, smem, tid, row, inner0, regs);
-  __syncthreads();
-  Inverse<N, T>::store(p, g, smem, tid, blockDim.x, row, inner0);
+  grid_dependency_wait();
+  with_operand(b, blockIdx.x, [&](const FftParams& p, const FftGeom& g, int tile, int tiles_x) {
+    const int row = tile / tiles_x;
+    const int inner0 = (tile - row * tiles_x) * T;
+    Forward<N, T>::load(p, g, smem, tid, blockDim.x, row, inner0);
+    __syncthreads();
+    LineRegs<N> regs;
+    Forward<N, T>::row_fetch(p, g, smem, tid, row, inner0, regs);
+    __syncthreads();  // the column buffer aliases the staged planes
+    Forward<N, T>::row_pass(g, smem, tid, regs);
+    __syncthreads();
+    Forward<N, T>::col_pass(p, g, smem, tid, row, inner0);
+  });
+}
+
+template <int N, int T, int OPS>
+__global__ void __launch_bounds__(block_threads<N, T>())
+fft2d_inverse_kernel(const __grid_constant__ FftBatch<OPS> b) {
+  extern __shared__ __align__(16) char smem[];
+  const int tid = threadIdx.x;
+  grid_dependency_wait();
+  if ((int)blockIdx.x < b.sum_blocks) {
+    row_sum_block(b.sum, blockIdx.x, smem);
+    return;
+  }
+  with_operand(b, (int)blockIdx.x - b.sum_blocks, [&](const FftParams& p, const FftGeom& g, int tile, int tiles_x) {
+    const int row = tile / tiles_x;
+    const int inner0 = (tile - row * tiles_x) * T;
+    Inverse<N, T>::col_pass(p, g, smem, tid, row, inner0);
+    __syncthreads();
+    LineRegs<N> regs;
+    Inverse<N, T>::row_fetch(g, smem, tid, regs);
+    __syncthreads();  // the staged output aliases the column buffer
+    Inverse<N, T>::row_pass(p, g, smem, tid, row, inner0, regs);
+    __syncthreads();
+    Inverse<N, T>::store(p, g, smem, tid, blockDim.x, row, inner0);
+  });
 }
 
 __device__ __forceinline__ void prefetch_l2(const void* p) {
   asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }
 
-template <int N, int T>
+// The persistent kernels look the operand up per tile (only small layers and the small operands of larger
+// ones reach the merged form): `tile` becomes the tile's number inside the operand.
+template <int OPS>
+__device__ __forceinline__ int operand_of_tile(const FftBatch<OPS>& b, int& tile) {
+  if constexpr (OPS == 1) {
+    return 0;
+  } else {
+    int op = 0;
+#pragma unroll
+    for (int i = 1; i < OPS; ++i)
+      if (tile >= b.tile_end[i - 1]) op = i;
+    if (op > 0) tile -= b.tile_end[op - 1];
+    return op;
+  }
+}
+
+template <int N, int T, int OPS>
 __global__ void __launch_bounds__(FBF_COOP_THREADS, 2)
-fft2d_forward_coop_kernel(const __grid_constant__ FftParams p, const __grid_constant__ FftGeom g) {
+fft2d_forward_coop_kernel(const __grid_constant__ FftBatch<OPS> b) {
   extern __shared__ __align__(16) char smem[];
   const int tid = threadIdx.x, nth = blockDim.x;
-  const int tiles_x = (p.kc + T - 1) / T;
-  const int total = tiles_x * p.n_rows;
+  const int total = b.tile_end[OPS - 1];
+  grid_dependency_wait();
   // persistent blocks: tile w, then w + gridDim.x, ...; the real planes of the next tile are
   // pulled into L2 while this one is transformed
   for (int w = blockIdx.x; w < total; w += gridDim.x) {
-  const int row = w / tiles_x;
-  const int inner0 = (w - row * tiles_x) * T;
-  if (w + (int)gridDim.x < total) {
-    const int wn = w + gridDim.x;
+  int tile = w;
+  const int op = operand_of_tile(b, tile);
+  const FftParams& p = b.p[op];
+  const FftGeom& g = b.g[op];
+  const int tiles_x = b.tiles_x[op];
+  const int row = tile / tiles_x;
+  const int inner0 = (tile - row * tiles_x) * T;
+  if (tile + (int)gridDim.x < tiles_x * p.n_rows) {
+    const int wn = tile + gridDim.x;
     const int rown = wn / tiles_x, innern = (wn - rown * tiles_x) * T;
     const long long plane_bytes = (long long)p.h * p.w * 4;
     for (int t = 0; t < T; ++t) {
@@ -140,18 +232,28 @@ fft2d_forward_coop_kernel(const __grid_constant__ FftParams p, const __grid_cons
   }
 }
 
-template <int N, int T>
+template <int N, int T, int OPS>
 __global__ void __launch_bounds__(FBF_COOP_THREADS, 2)
-fft2d_inverse_coop_kernel(const __grid_constant__ FftParams p, const __grid_constant__ FftGeom g) {
+fft2d_inverse_coop_kernel(const __grid_constant__ FftBatch<OPS> b) {
   extern __shared__ __align__(16) char smem[];
   const int tid = threadIdx.x, nth = blockDim.x;
-  const int tiles_x = (p.n_inner + T - 1) / T;
-  const int total = tiles_x * p.n_rows;
-  for (int w = blockIdx.x; w < total; w += gridDim.x) {
-  const int row = w / tiles_x;
-  const int inner0 = (w - row * tiles_x) * T;
-  if (p.spec_bin == 1 && w + (int)gridDim.x < total) {  // plane-major: the next tile's spectra are contiguous
-    const int wn = w + gridDim.x;
+  const int total = b.tile_end[OPS - 1];
+  grid_dependency_wait();
+  const int first = (int)blockIdx.x - b.sum_blocks, step = (int)gridDim.x - b.sum_blocks;
+  if (first < 0) {
+    row_sum_block(b.sum, blockIdx.x, smem);
+    return;
+  }
+  for (int w = first; w < total; w += step) {
+  int tile = w;
+  const int op = operand_of_tile(b, tile);
+  const FftParams& p = b.p[op];
+  const FftGeom& g = b.g[op];
+  const int tiles_x = b.tiles_x[op];
+  const int row = tile / tiles_x;
+  const int inner0 = (tile - row * tiles_x) * T;
+  if (p.spec_bin == 1 && tile + step < tiles_x * p.n_rows) {  // plane-major: the next tile's spectra are contiguous
+    const int wn = tile + step;
     const int rown = wn / tiles_x, innern = (wn - rown * tiles_x) * T;
     const long long plane_bytes = (long long)(N / 2 + 1) * N * 8;
     for (int t = 0; t < T; ++t) {
@@ -186,6 +288,7 @@ fft1d_forward_kernel(const __grid_constant__ FftParams p, const __grid_constant_
   extern __shared__ __align__(16) char smem[];
   const int tid = threadIdx.x, nth = blockDim.x;
   const int inner0 = blockIdx.x * T;
+  grid_dependency_wait();
   Forward<N, T>::load(p, g, smem, tid, nth, 0, inner0);
   __syncthreads();
   LineRegs<N> regs;
@@ -203,6 +306,7 @@ fft1d_inverse_kernel(const __grid_constant__ FftParams p, const __grid_constant_
   extern __shared__ __align__(16) char smem[];
   const int tid = threadIdx.x, nth = blockDim.x;
   const int inner0 = blockIdx.x * T;
+  grid_dependency_wait();
   Rows1D<N, T>::load_spectrum(p, g, smem, tid, nth, inner0);
   __syncthreads();
   LineRegs<N> regs;
@@ -213,100 +317,79 @@ fft1d_inverse_kernel(const __grid_constant__ FftParams p, const __grid_constant_
   Inverse<N, T>::store(p, g, smem, tid, nth, 0, inner0);
 }
 
-constexpr int kSmemMax = 227 * 1024;
-constexpr int kSmemTwoBlocks = 113 * 1024;
-
-constexpr bool tile_allowed(int N, int T) { return N > 32 ? T <= 8 : (N / 2 + 1) * T <= 512; }
-
-template <class GeomFn>
-int pick_tile(int N, GeomFn geom) {
-  int best_any = 0;
-  // 32-point transforms: 8 planes per block (more blocks per SM at 64-86 registers per thread) measured 5-10 %
-  // faster than 16; 8- and 16-point ones are fastest at 16
-  for (int T = (N == 32 ? 8 : 16); T >= 1; T >>= 1) {
-    if (!tile_allowed(N, T)) continue;
-    const int bytes = geom(T).smem_bytes;
-    if (bytes <= kSmemTwoBlocks) return T;
-    if (bytes <= kSmemMax && best_any == 0) best_any = T;
-  }
-  return best_any;
-}
+constexpr int kSmemTwoBlocks = 113 * 1024;  // shared memory of one of two resident blocks
 
 // Blocks of a persistent cooperative kernel: as many as are resident at once.
 int persistent_blocks(long long tiles, int smem_bytes) {
   const int sms = sm_count();
-  const int per_sm = smem_bytes <= kSmemTwoBlocks ? 2 : 1;
+  const int per_sm = smem_bytes <= kSmemTwoBlocks ? 2 : 1;  // any window at the tile sizes of fft_tile()
   const long long resident = (long long)sms * per_sm;
   return (int)(tiles < resident ? tiles : resident);
 }
 
-template <int N, int T>
-cudaError_t run_forward(const FftParams& p, cudaStream_t stream) {
-  if constexpr (!tile_allowed(N, T)) {
-    return cudaErrorInvalidConfiguration;
-  } else {
-    const FftGeom g = forward_geom(N, T, p.h, p.w, p.off_y, p.off_x);
-    void (*kernel)(FftParams, FftGeom);
-    if constexpr (N > 32) {
-      kernel = fft2d_forward_coop_kernel<N, T>;
-    } else {
-      if (g.threads != block_threads<N, T>()) return cudaErrorInvalidConfiguration;
-      kernel = fft2d_forward_kernel<N, T>;
-    }
-    cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), g.smem_bytes);
-    if (e != cudaSuccess) return e;
-    dim3 grid((p.kc + T - 1) / T, p.n_rows);
-    if constexpr (N > 32) grid = dim3(persistent_blocks((long long)grid.x * grid.y, g.smem_bytes), 1);
-    kernel<<<grid, g.threads, g.smem_bytes, stream>>>(p, g);
-    count_launch();
-    return cudaGetLastError();
-  }
+// The kernels address the spectrum with 32-bit element offsets.
+bool spectrum_fits(const FftParams& p, int N) {
+  const long long bins = (long long)(N / 2 + 1) * N;
+  return bins * p.n_rows * p.kc < (1LL << 31);
 }
 
-template <int N, int T>
-cudaError_t run_inverse(const FftParams& p, cudaStream_t stream) {
-  if constexpr (!tile_allowed(N, T)) {
-    return cudaErrorInvalidConfiguration;
-  } else {
-    const FftGeom g = inverse_geom(N, T, p.h, p.w);
-    void (*kernel)(FftParams, FftGeom);
-    if constexpr (N > 32) {
-      kernel = fft2d_inverse_coop_kernel<N, T>;
-    } else {
-      if (g.threads != block_threads<N, T>()) return cudaErrorInvalidConfiguration;
-      kernel = fft2d_inverse_kernel<N, T>;
+template <int N, int OPS>
+cudaError_t run_batch(bool inverse, const FftParams* ops, int count, const RowSum* sum, cudaStream_t stream) {
+  constexpr int T = fft_tile(N);
+  FftBatch<OPS> b{};
+  long long tiles = 0;
+  int smem = 0;
+  for (int i = 0; i < OPS; ++i) {
+    if (i < count) {
+      b.p[i] = ops[i];
+      b.g[i] = inverse ? inverse_geom(N, T, ops[i].h, ops[i].w)
+                       : forward_geom(N, T, ops[i].h, ops[i].w, ops[i].off_y, ops[i].off_x);
+      b.tiles_x[i] = ((inverse ? ops[i].n_inner : ops[i].kc) + T - 1) / T;
+      tiles += (long long)b.tiles_x[i] * ops[i].n_rows;
+      if (b.g[i].smem_bytes > smem) smem = b.g[i].smem_bytes;
     }
-    cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), g.smem_bytes);
-    if (e != cudaSuccess) return e;
-    dim3 grid((p.n_inner + T - 1) / T, p.n_rows);
-    if constexpr (N > 32) grid = dim3(persistent_blocks((long long)grid.x * grid.y, g.smem_bytes), 1);
-    kernel<<<grid, g.threads, g.smem_bytes, stream>>>(p, g);
-    count_launch();
-    return cudaGetLastError();
+    b.tile_end[i] = (int)tiles;
   }
+  if (tiles > 0x7fffffff) return cudaErrorInvalidConfiguration;
+  const int threads = b.g[0].threads;
+  if (sum && sum->rows > 0) {
+    b.sum = *sum;
+    b.sum_blocks = row_sum_blocks(*sum, threads);
+  }
+  void (*kernel)(FftBatch<OPS>);
+  long long blocks = tiles;
+  if constexpr (N > 32) {
+    kernel = inverse ? fft2d_inverse_coop_kernel<N, T, OPS> : fft2d_forward_coop_kernel<N, T, OPS>;
+    blocks = persistent_blocks(tiles, smem);
+  } else {
+    if (threads != block_threads<N, T>()) return cudaErrorInvalidConfiguration;
+    kernel = inverse ? fft2d_inverse_kernel<N, T, OPS> : fft2d_forward_kernel<N, T, OPS>;
+  }
+  cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
+  if (e != cudaSuccess) return e;
+  e = launch_dependent(kernel, dim3((unsigned)(blocks + b.sum_blocks)), threads, smem, stream, b);
+  count_launch();
+  return e;
 }
 
 template <int N>
-cudaError_t dispatch_tile(bool inverse, const FftParams& p, int T, cudaStream_t s) {
-  switch (T) {
-    case 1: return inverse ? run_inverse<N, 1>(p, s) : run_forward<N, 1>(p, s);
-    case 2: return inverse ? run_inverse<N, 2>(p, s) : run_forward<N, 2>(p, s);
-    case 4: return inverse ? run_inverse<N, 4>(p, s) : run_forward<N, 4>(p, s);
-    case 8: return inverse ? run_inverse<N, 8>(p, s) : run_forward<N, 8>(p, s);
-    case 16: return inverse ? run_inverse<N, 16>(p, s) : run_forward<N, 16>(p, s);
-  }
-  return cudaErrorInvalidConfiguration;
+cudaError_t run_ops(bool inverse, const FftParams* ops, int count, const RowSum* sum, cudaStream_t s) {
+  if (count == 1) return run_batch<N, 1>(inverse, ops, count, sum, s);
+  return run_batch<N, kMaxFftOps>(inverse, ops, count, sum, s);
 }
 
-cudaError_t dispatch(bool inverse, const FftParams& p, int N, int T, cudaStream_t s) {
+cudaError_t dispatch(bool inverse, const FftParams* ops, int count, const RowSum* sum, int N, cudaStream_t s) {
+  if (count < 1 || count > kMaxFftOps) return cudaErrorInvalidValue;
+  for (int i = 0; i < count; ++i)
+    if (ops[i].n_rows > 65535 || !spectrum_fits(ops[i], N)) return cudaErrorInvalidConfiguration;
   switch (N) {
-    case 2: return dispatch_tile<2>(inverse, p, T, s);
-    case 4: return dispatch_tile<4>(inverse, p, T, s);
-    case 8: return dispatch_tile<8>(inverse, p, T, s);
-    case 16: return dispatch_tile<16>(inverse, p, T, s);
-    case 32: return dispatch_tile<32>(inverse, p, T, s);
-    case 64: return dispatch_tile<64>(inverse, p, T, s);
-    case 128: return dispatch_tile<128>(inverse, p, T, s);
+    case 2: return run_ops<2>(inverse, ops, count, sum, s);
+    case 4: return run_ops<4>(inverse, ops, count, sum, s);
+    case 8: return run_ops<8>(inverse, ops, count, sum, s);
+    case 16: return run_ops<16>(inverse, ops, count, sum, s);
+    case 32: return run_ops<32>(inverse, ops, count, sum, s);
+    case 64: return run_ops<64>(inverse, ops, count, sum, s);
+    case 128: return run_ops<128>(inverse, ops, count, sum, s);
   }
   return cudaErrorInvalidValue;
 }
@@ -331,58 +414,26 @@ int sm_count() {
 void count_launch(int n) { g_launches.fetch_add(static_cast<uint64_t>(n), std::memory_order_relaxed); }
 uint64_t launch_count() { return g_launches.load(std::memory_order_relaxed); }
 
-int pick_forward_tile(int N, int h, int w, int pad_u, int pad_l) {
-  return pick_tile(N, [&](int T) { return forward_geom(N, T, h, w, pad_u, pad_l); });
-}
-int pick_inverse_tile(int N, int oh, int ow) {
-  return pick_tile(N, [&](int T) { return inverse_geom(N, T, oh, ow); });
+cudaError_t launch_forward(const FftParams* ops, int count, int N, cudaStream_t stream) {
+  return dispatch(false, ops, count, nullptr, N, stream);
 }
 
-// The kernels address the spectrum with 32-bit element offsets.
-bool spectrum_fits(const FftParams& p, int N) {
-  const long long bins = (long long)(N / 2 + 1) * N;
-  return bins * p.n_rows * p.kc < (1LL << 31);
-}
-
-cudaError_t launch_forward(const FftParams& p, int N, cudaStream_t stream) {
-  const int T = pick_forward_tile(N, p.h, p.w, p.off_y, p.off_x);
-  if (T == 0 || p.n_rows > 65535 || !spectrum_fits(p, N)) return cudaErrorInvalidConfiguration;
-  return dispatch(false, p, N, T, stream);
-}
-
-cudaError_t launch_inverse(const FftParams& p, int N, cudaStream_t stream) {
-  const int T = pick_inverse_tile(N, p.h, p.w);
-  if (T == 0 || p.n_rows > 65535 || !spectrum_fits(p, N)) return cudaErrorInvalidConfiguration;
-  return dispatch(true, p, N, T, stream);
+cudaError_t launch_inverse(const FftParams* ops, int count, const RowSum* sum, int N, cudaStream_t stream) {
+  return dispatch(true, ops, count, sum, N, stream);
 }
 
 namespace {
 
-template <int N, int T>
-cudaError_t run_1d(bool inverse, const FftParams& p, cudaStream_t stream) {
-  if constexpr (!tile_allowed(N, T)) {
-    return cudaErrorInvalidConfiguration;
-  } else {
-    const FftGeom g = inverse ? inverse_geom(N, T, p.h, p.w) : forward_geom(N, T, p.h, p.w, 0, p.off_x);
-    void (*kernel)(FftParams, FftGeom) = inverse ? fft1d_inverse_kernel<N, T> : fft1d_forward_kernel<N, T>;
-    cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), g.smem_bytes);
-    if (e != cudaSuccess) return e;
-    kernel<<<(p.n_inner + T - 1) / T, g.threads, g.smem_bytes, stream>>>(p, g);
-    count_launch();
-    return cudaGetLastError();
-  }
-}
-
 template <int N>
-cudaError_t dispatch_1d_tile(bool inverse, const FftParams& p, int T, cudaStream_t s) {
-  switch (T) {
-    case 1: return run_1d<N, 1>(inverse, p, s);
-    case 2: return run_1d<N, 2>(inverse, p, s);
-    case 4: return run_1d<N, 4>(inverse, p, s);
-    case 8: return run_1d<N, 8>(inverse, p, s);
-    case 16: return run_1d<N, 16>(inverse, p, s);
-  }
-  return cudaErrorInvalidConfiguration;
+cudaError_t run_1d(bool inverse, const FftParams& p, cudaStream_t stream) {
+  constexpr int T = fft_tile(N);
+  const FftGeom g = inverse ? inverse_geom(N, T, p.h, p.w) : forward_geom(N, T, p.h, p.w, 0, p.off_x);
+  void (*kernel)(FftParams, FftGeom) = inverse ? fft1d_inverse_kernel<N, T> : fft1d_forward_kernel<N, T>;
+  cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), g.smem_bytes);
+  if (e != cudaSuccess) return e;
+  e = launch_dependent(kernel, dim3((p.n_inner + T - 1) / T), g.threads, g.smem_bytes, stream, p, g);
+  count_launch();
+  return e;
 }
 
 }  // namespace
@@ -411,15 +462,13 @@ cudaError_t launch_fft1d(bool inverse, const float* real_in, float* real_out, fl
     p.kc = (int)planes;
     p.real_row_stride = 0;
     p.real_inner_stride = 1;
-    const int T = inverse ? pick_inverse_tile(N, h, n) : pick_forward_tile(N, h, n, 0, offset);
-    if (T == 0) return cudaErrorInvalidConfiguration;
     cudaError_t e;
     switch (N) {
-      case 2: e = dispatch_1d_tile<2>(inverse, p, T, stream); break;
-      case 4: e = dispatch_1d_tile<4>(inverse, p, T, stream); break;
-      case 8: e = dispatch_1d_tile<8>(inverse, p, T, stream); break;
-      case 16: e = dispatch_1d_tile<16>(inverse, p, T, stream); break;
-      case 32: e = dispatch_1d_tile<32>(inverse, p, T, stream); break;
+      case 2: e = run_1d<2>(inverse, p, stream); break;
+      case 4: e = run_1d<4>(inverse, p, stream); break;
+      case 8: e = run_1d<8>(inverse, p, stream); break;
+      case 16: e = run_1d<16>(inverse, p, stream); break;
+      case 32: e = run_1d<32>(inverse, p, stream); break;
       default: e = cudaErrorInvalidValue;
     }
     if (e != cudaSuccess) return e;
@@ -437,6 +486,7 @@ namespace {
 __global__ void __launch_bounds__(256)
 spectrum_to_reference_kernel(const float2* __restrict__ spec, float2* __restrict__ ref, long long planes, int kc,
                              int N, int transposed) {
+  grid_dependency_wait();
   const int KX = N / 2 + 1;
   const long long per_plane = (long long)KX * N;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < planes * per_plane;
@@ -467,6 +517,7 @@ spectrum_to_reference_kernel(const float2* __restrict__ spec, float2* __restrict
 __global__ void __launch_bounds__(256)
 reference_to_spectrum_kernel(const float2* __restrict__ ref, float2* __restrict__ spec, long long planes, int kc,
                              int N, int transposed) {
+  grid_dependency_wait();
   const int KX = N / 2 + 1;
   const long long bins = (long long)KX * N;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < bins * kc;
@@ -498,12 +549,10 @@ cudaError_t launch_spectrum_layout(bool to_reference, const float2* src, float2*
   const long long total = to_reference ? planes * (N / 2 + 1) * N : (long long)(N / 2 + 1) * N * kc;
   const long long want = (total + 255) / 256, cap = (long long)sm_count() * 16;
   const int blocks = (int)(want < 1 ? 1 : want < cap ? want : cap);
-  if (to_reference)
-    spectrum_to_reference_kernel<<<blocks, 256, 0, stream>>>(src, dst, planes, kc, N, transposed);
-  else
-    reference_to_spectrum_kernel<<<blocks, 256, 0, stream>>>(src, dst, planes, kc, N, transposed);
+  const cudaError_t e = launch_dependent(to_reference ? spectrum_to_reference_kernel : reference_to_spectrum_kernel,
+                                         dim3(blocks), 256, 0, stream, src, dst, planes, kc, N, (int)transposed);
   count_launch();
-  return cudaGetLastError();
+  return e;
 }
 
 }  // namespace fbfft

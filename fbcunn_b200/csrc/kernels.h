@@ -19,19 +19,57 @@ int sm_count();
 // already did (the attribute is per device and function; asking on every launch costs a driver call).
 cudaError_t ensure_dynamic_smem(const void* kernel, int bytes);
 
-// Largest plane tile (planes per block) whose shared memory fits, preferring two
-// resident blocks per SM; 0 when even one plane does not fit.
-int pick_forward_tile(int N, int h, int w, int pad_u, int pad_l);
-int pick_inverse_tile(int N, int oh, int ow);
+// ---- programmatic dependent launch -----------------------------------------------------------
+// Every kernel of a pass is launched so that its blocks may be placed, SM by SM, as the blocks of the kernel
+// before it leave, instead of after the last of them has gone: they do what needs no input and wait in
+// grid_dependency_wait() until that kernel has finished and its writes are visible.  Such a kernel calls
+// grid_dependency_wait() in every block before its first access to global memory (also when it only writes:
+// an earlier kernel may still be reading the buffer), which makes the order transitive along the stream.
+// No kernel here triggers its successor early (griddepcontrol.launch_dependents): successors placed beside
+// running blocks keep the shared-memory carve-out those were launched with, which leaves a transform almost no
+// L1 for its loads in flight -- the 32-point inverse of 131072 planes took 322 us behind a contraction that
+// triggered at its start, 226 us without -- and they cost the running kernel issue slots; measured slower on
+// every layer, the smallest too.  A step of 16 x 16 planes x 32 x 32: 60 us without this attribute, 43 with it.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-cudaError_t launch_forward(const FftParams& p, int N, cudaStream_t stream);
+template <class... Params, class... Args>
+cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, int threads, size_t smem_bytes, cudaStream_t stream,
+                             const Args&... args) {
+  cudaLaunchConfig_t config{};
+  config.gridDim = grid;
+  config.blockDim = dim3(threads);
+  config.dynamicSmemBytes = smem_bytes;
+  config.stream = stream;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = &attr;
+  config.numAttrs = 1;
+  return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+}
+
+// ---- transforms ------------------------------------------------------------------------------
+// dst[r] (=|+=) scale * sum_{i<count} src[r*ld + i*step], r < rows: the bias gradient, which rides in the
+// launch of the inverse transform of the same pass.
+struct RowSum {
+  const float* src;
+  float* dst;
+  int rows, count;
+  long long ld, step;
+  float scale;
+  int accumulate;
+};
+
+constexpr int kMaxFftOps = 3;
+// Transforms of up to kMaxFftOps operands in one launch (all of the same size N).
+cudaError_t launch_forward(const FftParams* ops, int count, int N, cudaStream_t stream);
+cudaError_t launch_inverse(const FftParams* ops, int count, const RowSum* sum, int N, cudaStream_t stream);
 // batched 1-D real <-> half-complex transforms of contiguous rows (the row phases of the 2-D kernels)
 cudaError_t launch_fft1d(bool inverse, const float* real_in, float* real_out, float2* spec, long long rows, int n,
                          int N, int offset, cudaStream_t stream);
 // The 1-D transforms of 64, 128 and 256 points (fft1d_lines.cu), same arguments.
 cudaError_t launch_fft1d_lines(bool inverse, const float* real_in, float* real_out, float2* spec, long long rows,
                                int n, int N, int offset, cudaStream_t stream);
-cudaError_t launch_inverse(const FftParams& p, int N, cudaStream_t stream);
 // Between the library's half spectrum [bin][plane (padded to kc)] and the reference's 2-D frequency
 // tensor (planes, N/2+1, N, 2) (nn.FFTWrapper, test/test_FFTModule.lua:310-342).
 cudaError_t launch_spectrum_layout(bool to_reference, const float2* src, float2* dst, long long planes, int kc, int N,
@@ -70,11 +108,10 @@ cudaError_t launch_bias_add(float* out, const float* bias, int batch, int planes
                             cudaStream_t stream);
 cudaError_t launch_bias_grad(const float* grad_out, float* grad_bias, float* scratch, int batch,
                              int planes, int hw, float scale, int accumulate, cudaStream_t stream);
-// dst[r] (=|+=) scale * sum_{i<count} src[r*ld + i*step]
 // dst[i] = src[i], or dst[i] += src[i]
 cudaError_t launch_copy_or_add(const float* src, float* dst, long long n, int accumulate, cudaStream_t stream);
-cudaError_t launch_row_sum(const float* src, float* dst, int rows, int count, long long ld, long long step,
-                           float scale, int accumulate, cudaStream_t stream);
+// The bias gradient in a launch of its own.
+cudaError_t launch_row_sum(const RowSum& p, cudaStream_t stream);
 
 // ---- sums across ranks over peer memory (peer.cu) ------------------------------------------
 constexpr int kMaxPeers = 8;  // the GPUs of one NVSwitch box

@@ -37,6 +37,7 @@ __global__ void __launch_bounds__(128) tiles_cut_kernel(const float* __restrict_
                                                         const __grid_constant__ TileGeom g) {
   const long long planes = (long long)g.B * g.nh * g.nw * g.C;
   const int per_plane = g.th * g.tw;
+  grid_dependency_wait();
   for (long long pl = blockIdx.x; pl < planes; pl += gridDim.x) {
     const int c = (int)(pl % g.C);
     const long long tile = pl / g.C;
@@ -64,6 +65,7 @@ __global__ void __launch_bounds__(256) tiles_gather_kernel(const float* __restri
   const long long planes = (long long)g.B * g.C;
   const int per_plane = g.H * g.W;
   const int tile_elems = g.th * g.tw;
+  grid_dependency_wait();
   for (long long pl = blockIdx.x; pl < planes; pl += gridDim.x) {
     const int c = (int)(pl % g.C);
     const long long b = pl / g.C;
@@ -91,16 +93,16 @@ __global__ void __launch_bounds__(256) tiles_gather_kernel(const float* __restri
 cudaError_t launch_cut(const float* image, float* tiles, const TileGeom& g, cudaStream_t s) {
   const long long planes = (long long)g.B * g.nh * g.nw * g.C;
   const long long cap = (long long)sm_count() * 64;
-  tiles_cut_kernel<<<(int)(planes < cap ? planes : cap), 128, 0, s>>>(image, tiles, g);
+  const cudaError_t e = launch_dependent(tiles_cut_kernel, dim3((unsigned)(planes < cap ? planes : cap)), 128, 0, s, image, tiles, g);
   count_launch();
-  return cudaGetLastError();
+  return e;
 }
 cudaError_t launch_gather(const float* tiles, float* image, const float* bias, const TileGeom& g, cudaStream_t s) {
   const long long planes = (long long)g.B * g.C;
   const long long cap = (long long)sm_count() * 32;
-  tiles_gather_kernel<<<(int)(planes < cap ? planes : cap), 256, 0, s>>>(tiles, image, bias, g);
+  const cudaError_t e = launch_dependent(tiles_gather_kernel, dim3((unsigned)(planes < cap ? planes : cap)), 256, 0, s, tiles, image, bias, g);
   count_launch();
-  return cudaGetLastError();
+  return e;
 }
 
 int ceil_div(int a, int b) { return (a + b - 1) / b; }

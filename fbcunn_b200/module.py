@@ -34,12 +34,23 @@ memoryReuseWeight = "weight"
 memoryReuseAll = "all"
 
 
-def _ptr(t: Optional[torch.Tensor]):
-    return ctypes.c_void_p(t.data_ptr()) if t is not None else None
+# Small layers are bound by what the host does per call: pointers and streams cross the boundary as plain
+# integers, and the handle of the last input shape is found by one comparison.
+def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
+    return t.data_ptr() if t is not None else None
 
 
-def _stream(device) -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+def _device_index(device: torch.device) -> int:
+    return device.index if device.index is not None else torch.cuda.current_device()
+
+
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
+    lambda index: torch.cuda.current_stream(index).cuda_stream)
+
+
+def _stream(device) -> int:
+    """The current stream of a device as the integer the C ABI takes."""
+    return _raw_stream(_device_index(device))
 
 
 def _is_number(x) -> bool:
@@ -109,6 +120,7 @@ class SpatialConvolutionFBFFT:
         self.reportErrors = True
         self._handle = None
         self._handle_key = None
+        self._out_shape = None
         self._comm = None
         self.reset()
 
@@ -126,25 +138,22 @@ class SpatialConvolutionFBFFT:
         self.timeSteps["updateOutput"] += 1
         self._check_input(input)
         h = self._prepare(input)
-        B, _, iH, iW = input.shape
-        oH, oW = iH + 2 * self.padUp - self.kH + 1, iW + 2 * self.padLeft - self.kW + 1
-        shape = (B, self.nOutputPlane, oH, oW)
-        if self.output is None or tuple(self.output.shape) != shape:
-            self.output = torch.empty(shape, dtype=torch.float32, device=self.device)
+        if self.output is None or self.output.shape != self._out_shape:
+            self.output = torch.empty(self._out_shape, dtype=torch.float32, device=self.device)
         capi.check(capi.lib().fbfftconv_update_output(
-            h, _ptr(input), _ptr(self.weight), None if skipBias else _ptr(self.bias),
-            _ptr(self.output), _stream(self.device)))
+            h, input.data_ptr(), self.weight.data_ptr(), None if skipBias else _ptr(self.bias),
+            self.output.data_ptr(), _stream(self.device)))
         return self.output
 
     def updateGradInput(self, input: torch.Tensor, gradOutput: torch.Tensor) -> torch.Tensor:
         self.timeSteps["updateGradInput"] += 1
         self._check_input(input)
-        self._check_grad_output(input, gradOutput)
         h = self._prepare(input)
+        self._check_grad_output(gradOutput)
         if self.gradInput is None or self.gradInput.shape != input.shape:
             self.gradInput = torch.empty_like(input)
         capi.check(capi.lib().fbfftconv_update_grad_input(
-            h, _ptr(gradOutput), _ptr(self.weight), _ptr(self.gradInput), _stream(self.device)))
+            h, gradOutput.data_ptr(), self.weight.data_ptr(), self.gradInput.data_ptr(), _stream(self.device)))
         return self.gradInput
 
     def accGradParameters(self, input: torch.Tensor, gradOutput: torch.Tensor, scale=None,
@@ -152,11 +161,11 @@ class SpatialConvolutionFBFFT:
         self.timeSteps["accGradParameters"] += 1
         scale = 1.0 if scale is None else float(scale)
         self._check_input(input)
-        self._check_grad_output(input, gradOutput)
         h = self._prepare(input)
+        self._check_grad_output(gradOutput)
         capi.check(capi.lib().fbfftconv_acc_grad_parameters(
-            h, _ptr(input), _ptr(gradOutput), _ptr(self.gradWeight),
-            None if skipBias else _ptr(self.gradBias), ctypes.c_float(scale), _stream(self.device)))
+            h, input.data_ptr(), gradOutput.data_ptr(), self.gradWeight.data_ptr(),
+            None if skipBias else _ptr(self.gradBias), scale, _stream(self.device)))
 
     # The per-pass implementations the reference's subclasses and wrappers call directly
     # (fbcunn/SpatialConvolutionFBFFT.lua:102, :189, :269; callers
@@ -177,9 +186,26 @@ class SpatialConvolutionFBFFT:
         return self.updateOutput(input)
 
     def backward(self, input, gradOutput, scale=None):
-        """updateGradInput then accGradParameters (fbcunn/SpatialConvolutionFFT.lua:405-416)."""
-        self.updateGradInput(input, gradOutput)
-        self.accGradParameters(input, gradOutput, scale)
+        """updateGradInput and accGradParameters (fbcunn/SpatialConvolutionFFT.lua:405-416) in one native
+        call, which transforms gradOutput once for both.  A subclass with passes of its own gets them
+        called one after the other."""
+        cls = type(self)
+        if (cls.updateGradInput is not SpatialConvolutionFBFFT.updateGradInput
+                or cls.accGradParameters is not SpatialConvolutionFBFFT.accGradParameters):
+            self.updateGradInput(input, gradOutput)
+            self.accGradParameters(input, gradOutput, scale)
+            return self.gradInput
+        self.timeSteps["updateGradInput"] += 1
+        self.timeSteps["accGradParameters"] += 1
+        self._check_input(input)
+        h = self._prepare(input)
+        self._check_grad_output(gradOutput)
+        if self.gradInput is None or self.gradInput.shape != input.shape:
+            self.gradInput = torch.empty_like(input)
+        capi.check(capi.lib().fbfftconv_backward(
+            h, input.data_ptr(), gradOutput.data_ptr(), self.weight.data_ptr(), self.gradInput.data_ptr(),
+            self.gradWeight.data_ptr(), self.gradBias.data_ptr(), 1.0 if scale is None else float(scale),
+            _stream(self.device)))
         return self.gradInput
 
     def zeroGradParameters(self):
@@ -243,12 +269,15 @@ class SpatialConvolutionFBFFT:
         assert input.dtype == torch.float32 and input.is_contiguous()
         assert input.shape[1] == self.nInputPlane, "num planes mismatch"
 
-    def _check_grad_output(self, input, gradOutput):
+    def _output_shape(self, input):
+        B, _, iH, iW = input.shape
+        return (B, self.nOutputPlane, iH + 2 * self.padUp - self.kH + 1, iW + 2 * self.padLeft - self.kW + 1)
+
+    def _check_grad_output(self, gradOutput):
+        """After _prepare, which knows the shape."""
         assert isinstance(gradOutput, torch.Tensor) and gradOutput.is_cuda, "CUDA support only!"
         assert gradOutput.dtype == torch.float32 and gradOutput.is_contiguous()
-        B, _, iH, iW = input.shape
-        oH, oW = iH + 2 * self.padUp - self.kH + 1, iW + 2 * self.padLeft - self.kW + 1
-        assert tuple(gradOutput.shape) == (B, self.nOutputPlane, oH, oW), "gradOutput size mismatch"
+        assert gradOutput.shape == self._out_shape, "gradOutput size mismatch"
 
     def _init_comm(self):
         uid, rank, nranks = self._comm
@@ -266,16 +295,15 @@ class SpatialConvolutionFBFFT:
 
     def _prepare(self, input):
         """prepareSizeAndBuffers: a native handle per (batch, image size)."""
-        B, _, iH, iW = input.shape
-        flags = self._flags()
-        key = (int(B), int(iH), int(iW), flags)
+        key = (input.shape, self._flags())
         if self._handle is not None and self._handle_key == key:
             return self._handle
         self.cleanupBuffers()
+        self._out_shape = self._output_shape(input)
+        (B, _, iH, iW), flags = key
         desc = capi.Desc(B, self.nInputPlane, self.nOutputPlane, iH, iW, self.kH, self.kW,
                          self.dH, self.dW, self.padUp, self.padLeft,
-                         self.device.index if self.device.index is not None else torch.cuda.current_device(),
-                         flags)
+                         _device_index(self.device), flags)
         h = ctypes.c_void_p()
         capi.check(capi.lib().fbfftconv_create(ctypes.byref(desc), ctypes.byref(h)))
         self._handle, self._handle_key = h, key
@@ -408,9 +436,9 @@ class FFTWrapper:
     def _scratch(self, planes, n_fft, device):
         """The library's own half spectrum of `planes` planes (a kernel converts it to / from the
         reference's tensor); kept between calls of the same size."""
-        need = int(capi.lib().fbfftconv_spectrum_bytes(n_fft, 1, planes))
+        need = (n_fft // 2 + 1) * n_fft * ((planes + 3) // 4 * 4) * 8  # fbfftconv_spectrum_bytes(n_fft, 1, planes)
         buf = getattr(self, "_scratch_buf", None)
-        if buf is None or buf.numel() < need or buf.device != torch.device(device):
+        if buf is None or buf.numel() < need or buf.device != device:
             buf = torch.empty(need, dtype=torch.uint8, device=device)
             self._scratch_buf = buf
         return buf

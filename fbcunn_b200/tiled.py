@@ -24,7 +24,7 @@ import ctypes
 import torch
 
 from . import capi
-from .module import SpatialConvolutionFBFFT, _ptr, _stream
+from .module import SpatialConvolutionFBFFT, _device_index, _ptr, _stream
 
 
 class SpatialConvolutionFFTTiled(SpatialConvolutionFBFFT):
@@ -55,15 +55,15 @@ class SpatialConvolutionFFTTiled(SpatialConvolutionFBFFT):
         return oH, oW, tH, tW, sH, sW, nH, nW, pH, pW
 
     def _prepare_tiled(self, input):
-        B, _, iH, iW = input.shape
-        flags = self._flags()
-        key = (int(B), int(iH), int(iW), flags)
+        key = (input.shape, self._flags())
         if self._tiled is not None and self._tiled_key == key:
             return self._tiled
         self.cleanupBuffers()
+        self._out_shape = self._output_shape(input)
+        (B, _, iH, iW), flags = key
         desc = capi.Desc(B, self.nInputPlane, self.nOutputPlane, iH, iW, self.kH, self.kW, self.dH, self.dW,
                          self.padUp, self.padLeft,
-                         self.device.index if self.device.index is not None else torch.cuda.current_device(), flags)
+                         _device_index(self.device), flags)
         t = ctypes.c_void_p()
         capi.check(capi.lib().fbfftconv_tiled_create(ctypes.byref(desc), self.tileSizeH, self.tileSizeW,
                                                      ctypes.byref(t)))
@@ -80,11 +80,8 @@ class SpatialConvolutionFFTTiled(SpatialConvolutionFBFFT):
         self.timeSteps["updateOutput"] += 1
         self._check_input(input)
         t = self._prepare_tiled(input)
-        B, _, iH, iW = input.shape
-        oH, oW = self._geometry(iH, iW)[:2]
-        shape = (B, self.nOutputPlane, oH, oW)
-        if self.output is None or tuple(self.output.shape) != shape:
-            self.output = torch.empty(shape, dtype=torch.float32, device=self.device)
+        if self.output is None or self.output.shape != self._out_shape:
+            self.output = torch.empty(self._out_shape, dtype=torch.float32, device=self.device)
         capi.check(capi.lib().fbfftconv_tiled_update_output(
             t, _ptr(input), _ptr(self.weight), None if skipBias else _ptr(self.bias), _ptr(self.output),
             _stream(self.device)))
@@ -93,8 +90,8 @@ class SpatialConvolutionFFTTiled(SpatialConvolutionFBFFT):
     def updateGradInput(self, input: torch.Tensor, gradOutput: torch.Tensor) -> torch.Tensor:
         self.timeSteps["updateGradInput"] += 1
         self._check_input(input)
-        self._check_grad_output(input, gradOutput)
         t = self._prepare_tiled(input)
+        self._check_grad_output(gradOutput)
         if self.gradInput is None or self.gradInput.shape != input.shape:
             self.gradInput = torch.empty_like(input)
         capi.check(capi.lib().fbfftconv_tiled_update_grad_input(
@@ -106,8 +103,8 @@ class SpatialConvolutionFFTTiled(SpatialConvolutionFBFFT):
         self.timeSteps["accGradParameters"] += 1
         scale = 1.0 if scale is None else float(scale)
         self._check_input(input)
-        self._check_grad_output(input, gradOutput)
         t = self._prepare_tiled(input)
+        self._check_grad_output(gradOutput)
         capi.check(capi.lib().fbfftconv_tiled_acc_grad_parameters(
             t, _ptr(input), _ptr(gradOutput), _ptr(self.gradWeight), None if skipBias else _ptr(self.gradBias),
             ctypes.c_float(scale), _stream(self.device)))

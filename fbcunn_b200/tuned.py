@@ -168,8 +168,9 @@ class SpatialConvolution:
         return self.updateOutput(input)
 
     def backward(self, input, gradOutput, scale=None):
-        self.updateGradInput(input, gradOutput)
-        self.accGradParameters(input, gradOutput, scale)
+        assert self.bestModuleInst is not None, "updateOutput runs first (it tunes)"
+        assert not self.inferenceOnly, "module was built for inference only"
+        self.gradInput = self.bestModuleInst.backward(input, gradOutput, scale)
         return self.gradInput
 
     def zeroGradParameters(self):

@@ -136,6 +136,14 @@ int fbfftconv_acc_grad_parameters(fbfftconv_handle* h, const float* input, const
                                   float* grad_weight, float* grad_bias, float scale,
                                   fbfftconv_stream stream);
 
+/* nn.Module:backward(input, gradOutput, scale) (fbcunn/SpatialConvolutionFFT.lua:405-416):
+ * updateGradInput and accGradParameters in one call, with gradOutput, which both see unchanged,
+ * transformed once.  The results are those of the two calls.  grad_input must not overlap input,
+ * grad_output or weight. */
+int fbfftconv_backward(fbfftconv_handle* h, const float* input, const float* grad_output, const float* weight,
+                       float* grad_input, float* grad_weight, float* grad_bias, float scale,
+                       fbfftconv_stream stream);
+
 /* ---- the same passes on tiles of the image -----------------------------------
  * Replaces nn.SpatialConvolutionFFTTiled (fbcunn/SpatialConvolutionFFTTiled.lua:265-365, :489-563,
  * :601-683, :724-802): the output is cut into disjoint tiles of (tile - k + 1) pixels, each computed
@@ -365,9 +373,8 @@ enum {
 int fbfftconv_profile_enable(fbfftconv_handle* h, int enable);
 int fbfftconv_profile_reset(fbfftconv_handle* h);
 int fbfftconv_profile_read(fbfftconv_handle* h, int pass, int stage, double* total_ms, int* launches);
-/* 1 if launches of this stage since the last reset ran next to another stage of the pass on the
- * handle's second stream (a small second forward transform): its time then overlaps the other
- * stage's and is not its cost alone.  0 otherwise, negative on a bad query. */
+/* Kept for callers of earlier versions: kernels that are timed run one after the other on the caller's
+ * stream, so the answer is 0 (-1 for a bad query). */
 int fbfftconv_profile_overlapped(const fbfftconv_handle* h, int pass, int stage);
 
 /* ---- diagnostics ------------------------------------------------------------ */

@@ -222,13 +222,12 @@ struct FftGeom {
   int N, T;
   int he, we;      // forward: extent of the data inside the N x N square (offset included);
                    // inverse: the crop window
-  int hh;          // row pairs: rows (j, j + hh) share one complex line
+  int hh;          // row pairs that share one complex line: rows (j, j + hh); cooperative: (2j, 2j + 1)
   int hh_magic;    // ceil(2^16 / hh): line / hh == (line * hh_magic) >> 16 for line < 512, hh <= 64
-  int pitch1;      // cooperative: line pitch of the row buffer; thread-per-line: pitch of a staged real plane (floats)
+  int pitch1;      // thread-per-line: pitch of a staged real plane (floats)
   int pitch2;      // row pitch of the column buffer ("mid")
   int lines1;      // hh * T
   int lines2;      // (N/2 + 1) * T
-  int chunk;       // cooperative kernels: row lines processed per round
   int threads;
   int off_a, off_b;  // byte offsets of the two shared-memory regions
   int smem_bytes;
@@ -239,16 +238,22 @@ static inline bool cooperative(int N) { return N > 32; }
 // 5-10 % faster than 16); 8- and 16-point ones are fastest at 16; the cooperative sizes take what lets two
 // blocks share an SM's memory.
 constexpr int fft_tile(int N) { return N > 64 ? 1 : N > 32 ? 4 : N > 16 ? 8 : 16; }
-#define FBF_COOP_THREADS 256  // measured slower: 288 (whole rounds in the column phases, but a 96-register cap), 384, 512
-static_assert(FBF_COOP_THREADS % 32 == 0, "whole warps, and a multiple of every N2");
-static inline int coop_threads() { return FBF_COOP_THREADS; }
+// Threads of a cooperative block and blocks per SM.  With the column buffer alone in shared memory (69 / 74 KB)
+// three blocks fit an SM, but what bounds these kernels is instruction issue and the latency of a thread's own
+// chain: below 128 registers (three blocks of 192 or 256 threads) spills through the little L1 that is left cost
+// more than the extra warps bring.  Step of a first layer (128 x 3 -> 96 planes of 128 x 128) and of a 64-pixel
+// layer (128 x 64 -> 128 planes), us: 160 x 3 1572 / 1396, 192 x 2 1584 / 1269, 256 x 2 1594 / 1256, 128 x 3
+// 1597 / 1399, 192 x 3 1771 / 1356, 256 x 3 2063 / 1340 (two blocks of 256 threads with a row buffer and block
+// barriers between the row steps: 1626 / 1320; this choice per size: 1556 / 1261).
+constexpr int coop_threads(int N) { return N > 64 ? 160 : 256; }
+constexpr int coop_blocks(int N) { return N > 64 ? 3 : 2; }
 
 // Thread-per-line kernels (N <= 32): region A = the T real planes as they lie in global
 // memory (pitch1 floats apart), region B = column buffer [y][kx*T + t]; they alias (a thread
 // takes its whole line into registers before the barrier that precedes the first write of the
 // other region).
-// Cooperative kernels (N > 32): region A = one chunk of row lines
-// [line][k1*(N2+1) + n2], region B = column buffer [y or slot][t*(N/2+1) + kx].
+// Cooperative kernels (N > 32): one column buffer [y or slot][t*KXP + kx]; a row line passes
+// through the two rows of it that it will fill (CoopLayout::line_slot).
 // Pitch (floats) of one staged real plane of n elements: a multiple of 4 (16-byte copies)
 // with room for the 0..3 floats by which a plane is shifted to share the 16-byte phase of
 // its global address, and an odd number of 16-byte units so that neighbouring planes start
@@ -259,10 +264,10 @@ static inline int stage_pitch(int n) {
   return p;
 }
 
-// Row pitch (float2) of the cooperative kernels' column buffer: at least `cols`, and 8 modulo 16, so that
-// the eight-element runs that the lanes of neighbouring row lines store in one instruction (row step 2)
-// fall into different halves of the banks.  The column phases walk along the rows and do not care.
-constexpr int coop_mid_pitch(int cols) { return (cols + 7) / 16 * 16 + 8; }
+// Row pitch (float2) of the cooperative kernels' column buffer: at least `cols`, and 4 modulo 16.  A row line
+// occupies two neighbouring rows and the lines that share an access are two rows apart, so their runs of four
+// (128 points) or eight (64 points) values fall on different banks in both row steps.
+constexpr int coop_mid_pitch(int cols) { return (cols + 11) / 16 * 16 + 4; }
 // Distance (float2) between the planes of a tile inside a row of the column buffer: N/2 + 1 values per
 // plane, spaced 4 modulo 16 apart when a tile has several planes, so that the lanes that take the T
 // planes of neighbouring bins (column step 2 of the forward, column step 1 of the inverse) use
@@ -284,22 +289,17 @@ static inline FftGeom make_geom(int N, int T, int he, int we, int plane_elems, b
   if (!cooperative(N)) {
     g.pitch1 = stage_pitch(plane_elems);
     g.pitch2 = plane_pitch(g.lines2, T);
-    g.chunk = g.lines1;
     const int bytes_a = T * g.pitch1 * 4;
     const int bytes_b = he * g.pitch2 * 8;
     g.off_b = 0;
     g.smem_bytes = bytes_a > bytes_b ? bytes_a : bytes_b;
     g.threads = round_up(g.lines2 < 64 ? 64 : g.lines2, 32);
   } else {
-    const int n1 = N == 64 ? 8 : 8, n2 = N / n1;
-    g.pitch1 = n1 * (n2 + 1);          // = CoopLayout::PITCH1
+    g.pitch1 = 0;
     g.pitch2 = coop_mid_pitch(T * coop_plane_stride(N / 2 + 1, T));  // = CoopLayout::PITCH2
-    g.chunk = N == 64 ? 64 : 32;
-    if (g.chunk > g.lines1) g.chunk = g.lines1;
-    const int bytes_a = g.chunk * g.pitch1 * 8;
-    g.off_b = round_up(bytes_a, 16);
-    g.smem_bytes = g.off_b + N * g.pitch2 * 8;
-    g.threads = coop_threads();
+    g.off_b = 0;
+    g.smem_bytes = N * g.pitch2 * 8;
+    g.threads = coop_threads(N);
   }
   return g;
 }
@@ -614,13 +614,18 @@ struct CoopLayout {
       return col + t * (KXP - KX);
     }
   }
-  // Row buffer line pitch (float2): 72 / 136, i.e. 8 modulo 16.  In the second row step the eight lanes of
-  // a line read at a stride of N2 + 1 and cover half of the banks; the next line's lanes, 16 banks on, the
-  // other half.  (The first row step stores 8 or 16 neighbouring values per line and does not care.)
-  static constexpr int PITCH1 = N1 * (N2 + 1);
-  static_assert(PITCH1 % 16 == 8, "neighbouring lines of the second row step: different halves of the banks");
   static constexpr int PITCH2 = coop_mid_pitch(T * KXP);  // mid row pitch (float2)
   static_assert(N1 == 8, "the residue pairing below is written for eight residues");
+  static_assert(coop_threads(N) % 32 == 0, "whole warps");
+  // Between its two steps a row line lies where its result goes: values (k1, n2) of residues 0-3 in the plane's
+  // part of the pair's first row, those of residues 4-7 in the second row.  A line then belongs to one warp
+  // from its loads to its last store: no row buffer, no block barrier between the row steps, and the shared
+  // memory of a block is the column buffer alone.
+  static constexpr int HALF = 4 * (N2 + 1);
+  static_assert(HALF <= (T == 1 ? PITCH2 : KXP), "half a line fits a plane's part of a row");
+  static FBF_HD int slot_in_half(int k1) { return (k1 & 3) * (N2 + 1); }
+  // Lines that a warp takes at a time: two items of the first row step per lane.
+  static constexpr int TASK_LINES = 64 / N2;
 };
 
 // Order of the residues k1 inside a group of eight neighbouring lanes: residues that
@@ -649,92 +654,92 @@ struct CoopForward {
 
   struct RowLoad {
     float2 v[N1];
-    int slot;  // ll * PITCH1 + n2, or -1
-    int n2;
+    int slot;  // mid element of value (k1 = 0, n2) of the line, or -1
   };
 
+  // Item `item` of the first row step of the lines line0 .. line0 + TASK_LINES - 1 (one warp's task): the
+  // rows (2j, 2j + 1) of a plane at columns n2 + N2*n1.
   static FBF_HD void row_fetch(const FftParams& p, const FftGeom& g, const float* base, long long tstride,
-                               int inner0, int line0, int nl, int item, RowLoad& r) {
-    r.slot = -1;
-    if (item >= nl * N2) return;
+                               int inner0, int line0, int item, RowLoad& r) {
     const int ll = item / N2, n2 = item - ll * N2;
     const int line = line0 + ll;
+    r.slot = -1;
+    if (line >= g.lines1) return;
     int t, j;
     coop_split_line<T>(g, line, t, j);
     const bool live = inner0 + t < p.n_inner;
     const float* plane = base + t * tstride;
-    const int ya = j - p.off_y, yb = j + g.hh - p.off_y;
+    const int ya = 2 * j - p.off_y, yb = ya + 1;
     const bool va = live && ya >= 0 && ya < p.h, vb = live && yb >= 0 && yb < p.h;
     const float* pa = plane + ya * p.w + (n2 - p.off_x);
-    const float* pb = plane + yb * p.w + (n2 - p.off_x);
+    const float* pb = pa + p.w;
 #pragma unroll
     for (int n1 = 0; n1 < N1; ++n1) {
       const int x = N2 * n1 + n2 - p.off_x;
       const bool vx = x >= 0 && x < p.w;
       r.v[n1] = make_float2(va && vx ? pa[N2 * n1] : 0.f, vb && vx ? pb[N2 * n1] : 0.f);
     }
-    r.slot = ll * L::PITCH1 + n2;
-    r.n2 = n2;
+    r.slot = 2 * j * L::PITCH2 + t * L::KXP + n2;
   }
 
-  static FBF_HD void row_transform(float2* rb, RowLoad& r, const float2 (&tw)[N1]) {
+  static FBF_HD void row_transform(float2* mid, RowLoad& r, const float2 (&tw)[N1]) {
     if (r.slot < 0) return;
     fft_inreg<N1, false>(r.v);
-    float2* dst = rb + r.slot;
+    float2* dst = mid + r.slot;
     dst[0] = r.v[0];
 #pragma unroll
-    for (int k1 = 1; k1 < N1; ++k1) dst[k1 * (N2 + 1)] = cmul(r.v[k1], tw[k1]);
+    for (int k1 = 1; k1 < N1; ++k1) dst[(k1 >> 2) * L::PITCH2 + L::slot_in_half(k1)] = cmul(r.v[k1], tw[k1]);
   }
 
-  // Row step 1 for lines [line0, line0 + nl): straight from global memory (N2
-  // neighbouring floats per row and lane group: whole 32-byte sectors), two items in
-  // flight per thread, N1-point transform, twiddle, into the row buffer.
-  static FBF_HD void row_step1(const FftParams& p, const FftGeom& g, char* smem, int tid, int nthreads,
-                               int row, int inner0, int line0, int nl) {
-    float2* rb = reinterpret_cast<float2*>(smem + g.off_a);
+  static FBF_HD void row_twiddles(int lane, float2 (&tw)[N1]) {
+#pragma unroll
+    for (int k1 = 0; k1 < N1; ++k1) tw[k1] = tw128_runtime<false>((lane % N2) * k1 * (128 / N));
+  }
+
+  // Row step 1 of a warp's task: straight from global memory (N2 neighbouring floats per row and lane
+  // group: whole 32-byte sectors), two items in flight per lane, N1-point transform, twiddle, into mid.
+  static FBF_HD void row_step1(const FftParams& p, const FftGeom& g, char* smem, int lane, int row, int inner0,
+                               int line0, const float2 (&tw)[N1]) {
+    float2* mid = reinterpret_cast<float2*>(smem + g.off_b);
     const long long plane_elems = (long long)p.h * p.w;
     const float* base = p.real_in + (row * p.real_row_stride + inner0 * p.real_inner_stride) * plane_elems;
     const long long tstride = p.real_inner_stride * plane_elems;
-    // the block size is a multiple of N2, so a thread meets the same n2 in all its items
-    float2 tw[N1];
-#pragma unroll
-    for (int k1 = 0; k1 < N1; ++k1) tw[k1] = tw128_runtime<false>((tid % N2) * k1 * (128 / N));
-    for (int item = tid; item < nl * N2; item += 2 * nthreads) {
-      RowLoad r0, r1;
-      row_fetch(p, g, base, tstride, inner0, line0, nl, item, r0);
-      row_fetch(p, g, base, tstride, inner0, line0, nl, item + nthreads, r1);
-      row_transform(rb, r0, tw);
-      row_transform(rb, r1, tw);
-    }
+    RowLoad r0, r1;
+    row_fetch(p, g, base, tstride, inner0, line0, lane, r0);
+    row_fetch(p, g, base, tstride, inner0, line0, lane + 32, r1);
+    row_transform(mid, r0, tw);
+    row_transform(mid, r1, tw);
   }
 
   // Row step 2, first half: item = (line, lane position); the N2-point transform of
   // residue k1 of that line.
-  static FBF_HD bool row_step2_fft(const FftGeom& g, const char* smem, int item, int nl, float2 (&u)[N2]) {
-    if (item >= nl * N1) return false;
-    const float2* rb = reinterpret_cast<const float2*>(smem + g.off_a);
-    const int ll = item / N1, k1 = coop_residue_of_lane(item % N1);
-    const float2* src = rb + ll * L::PITCH1 + k1 * (N2 + 1);
+  static FBF_HD bool row_step2_fft(const FftGeom& g, const char* smem, int line0, int item, float2 (&u)[N2]) {
+    const int line = line0 + item / N1, k1 = coop_residue_of_lane(item % N1);
+    if (line >= g.lines1) return false;
+    int t, j;
+    coop_split_line<T>(g, line, t, j);
+    const float2* src = reinterpret_cast<const float2*>(smem + g.off_b) + (2 * j + (k1 >> 2)) * L::PITCH2 +
+                        t * L::KXP + L::slot_in_half(k1);
 #pragma unroll
     for (int n2 = 0; n2 < N2; ++n2) u[n2] = src[n2];
     fft_inreg<N2, false>(u);
     return true;
   }
 
-  // Row step 2, second half: Z[k] (own) meets Z[N-k] (own for residues 0 and N1/2, else
-  // the odd-indexed outputs of the mirror residue, handed over by the neighbouring
-  // lane); the row pair is split and written to mid.  Each lane of a mirror pair takes
-  // the even-indexed half of its own outputs, which covers every frequency once.
-  static FBF_HD void row_step2_split(const FftGeom& g, char* smem, int item, int line0,
+  // Row step 2, second half (after every lane of the warp has read its part of the line, which the
+  // result overwrites): Z[k] (own) meets Z[N-k] (own for residues 0 and N1/2, else the odd-indexed
+  // outputs of the mirror residue, handed over by the neighbouring lane); the row pair is split and
+  // written to mid.  Each lane of a mirror pair takes the even-indexed half of its own outputs, which
+  // covers every frequency once.
+  static FBF_HD void row_step2_split(const FftGeom& g, char* smem, int line0, int item,
                                      const float2 (&u)[N2], const float2 (&mirror_odd)[N2 / 2]) {
     float2* mid = reinterpret_cast<float2*>(smem + g.off_b);
-    const int ll = item / N1, k1 = coop_residue_of_lane(item % N1);
-    const int line = line0 + ll;
+    const int line = line0 + item / N1, k1 = coop_residue_of_lane(item % N1);
     int t, j;
     coop_split_line<T>(g, line, t, j);
-    const bool has_b = (j + g.hh) < g.he;
-    float2* ma = mid + j * L::PITCH2 + t * L::KXP;
-    float2* mb = mid + (j + g.hh) * L::PITCH2 + t * L::KXP;
+    const bool has_b = 2 * j + 1 < g.he;
+    float2* ma = mid + 2 * j * L::PITCH2 + t * L::KXP;
+    float2* mb = ma + L::PITCH2;
     if (k1 == 0 || k1 == N1 / 2) {
 #pragma unroll
       for (int k2 = 0; k2 <= N2 / 2; ++k2) {
@@ -887,66 +892,85 @@ struct CoopInverse {
     }
   }
 
-  // Row step 1 for lines [line0, line0+nl): rows (y0+j, y0+j+hh) of mid become one complex
-  // line (Hermitian extension), N1-point inverse transform, twiddle, into the row buffer.
-  static FBF_HD void row_step1(const FftParams& p, const FftGeom& g, char* smem, int tid, int nthreads,
-                               int line0, int nl) {
-    float2* rb = reinterpret_cast<float2*>(smem + g.off_a);
+  static FBF_HD void row_twiddles(int lane, float2 (&tw)[N1]) {
+#pragma unroll
+    for (int k1 = 0; k1 < N1; ++k1) tw[k1] = tw128_runtime<true>((lane % N2) * k1 * (128 / N));
+  }
+  // Elements of mid where the first and second row of line (t, j) begin.  The partner of an odd last row
+  // is a row outside the crop: the next one, or -- the crop ends with the square, at an odd offset then --
+  // the one before the crop.
+  static FBF_HD void line_rows(const FftParams& p, const FftGeom& g, int t, int j, int& ra, int& rb) {
+    const int ya = p.off_y + 2 * j;
+    const int yb = ya + 1 < N ? ya + 1 : p.off_y - 1;
+    ra = ya * L::PITCH2 + t * L::KXP;
+    rb = yb * L::PITCH2 + t * L::KXP;
+  }
+
+  // Row step 1, first half: item of the lines line0 .. line0 + TASK_LINES - 1 (one warp's task): the rows
+  // of mid become one complex line (Hermitian extension), N1-point inverse transform.
+  static FBF_HD bool row_step1_fft(const FftParams& p, const FftGeom& g, const char* smem, int line0, int item,
+                                   float2 (&v)[N1]) {
     const float2* mid = reinterpret_cast<const float2*>(smem + g.off_b);
-    // the block size is a multiple of N2, so a thread meets the same n2 in all its items
-    float2 tw[N1];
-#pragma unroll
-    for (int k1 = 0; k1 < N1; ++k1) tw[k1] = tw128_runtime<true>((tid % N2) * k1 * (128 / N));
-    for (int item = tid; item < nl * N2; item += nthreads) {
-      const int ll = item / N2, n2 = item - ll * N2;
-      const int line = line0 + ll;
-      int t, j;
+    const int ll = item / N2, n2 = item - ll * N2;
+    const int line = line0 + ll;
+    if (line >= g.lines1) return false;
+    int t, j, ra, rb;
     coop_split_line<T>(g, line, t, j);
-      const bool has_b = (j + g.hh) < g.he;
-      const float2* pa = mid + (p.off_y + j) * L::PITCH2 + t * L::KXP;
-      const float2* pb = pa + g.hh * L::PITCH2;
-      float2 v[N1];
+    line_rows(p, g, t, j, ra, rb);
+    const bool has_b = 2 * j + 1 < g.he;
+    const float2 *pa = mid + ra, *pb = mid + rb;
 #pragma unroll
-      for (int n1 = 0; n1 < N1; ++n1) {
-        const int k = N2 * n1 + n2;
-        const int kk = k <= N / 2 ? k : N - k;
-        const float2 a = pa[kk];
-        const float2 b = has_b ? pb[kk] : make_float2(0.f, 0.f);
-        v[n1] = k <= N / 2 ? tangle_low(a, b) : tangle_high(a, b);
-      }
-      fft_inreg<N1, true>(v);
-      float2* dst = rb + ll * L::PITCH1 + n2;
-      dst[0] = v[0];
-#pragma unroll
-      for (int k1 = 1; k1 < N1; ++k1) dst[k1 * (N2 + 1)] = cmul(v[k1], tw[k1]);
+    for (int n1 = 0; n1 < N1; ++n1) {
+      const int k = N2 * n1 + n2;
+      const int kk = k <= N / 2 ? k : N - k;
+      const float2 a = pa[kk];
+      const float2 b = has_b ? pb[kk] : make_float2(0.f, 0.f);
+      v[n1] = k <= N / 2 ? tangle_low(a, b) : tangle_high(a, b);
     }
+    fft_inreg<N1, true>(v);
+    return true;
+  }
+
+  // Row step 1, second half (after the warp has read the rows): twiddle, back into the line's rows.
+  static FBF_HD void row_step1_store(const FftParams& p, const FftGeom& g, char* smem, int line0, int item,
+                                     const float2 (&v)[N1], const float2 (&tw)[N1]) {
+    float2* mid = reinterpret_cast<float2*>(smem + g.off_b);
+    const int ll = item / N2, n2 = item - ll * N2;
+    int t, j, ra, rb;
+    coop_split_line<T>(g, line0 + ll, t, j);
+    line_rows(p, g, t, j, ra, rb);
+    float2 *da = mid + ra + n2, *db = mid + rb + n2;
+    da[0] = v[0];
+#pragma unroll
+    for (int k1 = 1; k1 < N1; ++k1) (k1 < 4 ? da : db)[L::slot_in_half(k1)] = cmul(v[k1], tw[k1]);
   }
 
   // Row step 2: item (line, k1) produces x = k1 + N1*k2 of both rows of the pair and
   // writes the crop columns straight to global memory (N1 neighbouring floats per row and
   // lane group: whole 32-byte sectors), bias added.
-  static FBF_HD void row_step2(const FftParams& p, const FftGeom& g, const char* smem, int tid,
-                               int nthreads, int row, int inner0, int line0, int nl) {
-    const float2* rb = reinterpret_cast<const float2*>(smem + g.off_a);
+  static FBF_HD void row_step2(const FftParams& p, const FftGeom& g, const char* smem, int row, int inner0,
+                               int line0, int item) {
+    const float2* mid = reinterpret_cast<const float2*>(smem + g.off_b);
     const long long plane_elems = (long long)g.he * g.we;
     float* base = p.real_out + (row * p.real_row_stride + inner0 * p.real_inner_stride) * plane_elems;
     const long long tstride = p.real_inner_stride * plane_elems;
-    for (int item = tid; item < nl * N1; item += nthreads) {
-      const int ll = item / N1, k1 = item - ll * N1;
-      const int line = line0 + ll;
-      int t, j;
-    coop_split_line<T>(g, line, t, j);
+    {
+      const int line = line0 + item / N1, k1 = item % N1;
+      if (line >= g.lines1) return;
+      int t, j, ra, rb;
+      coop_split_line<T>(g, line, t, j);
+      line_rows(p, g, t, j, ra, rb);
       const int inner = inner0 + t;
-      if (inner >= p.n_inner) continue;
-      const bool has_b = (j + g.hh) < g.he;
-      const float2* src = rb + ll * L::PITCH1 + k1 * (N2 + 1);
+      if (inner >= p.n_inner) return;
+      const bool has_b = 2 * j + 1 < g.he;
+      const float2* src = mid + (k1 < 4 ? ra : rb) + L::slot_in_half(k1);
       float2 u[N2];
 #pragma unroll
       for (int n2 = 0; n2 < N2; ++n2) u[n2] = src[n2];
       fft_inreg<N2, true>(u);
       const float bias = p.bias ? p.bias[p.bias_by_row ? row : inner] : 0.f;
-      float* da = base + t * tstride + (long long)j * g.we + (k1 - p.off_x);
-      float* db = da + (long long)g.hh * g.we;
+      float* da = base + t * tstride + (long long)(2 * j) * g.we + (k1 - p.off_x);
+      float* db = da + g.we;
 #pragma unroll
       for (int k2 = 0; k2 < N2; ++k2) {
         const int x = k1 + N1 * k2 - p.off_x;

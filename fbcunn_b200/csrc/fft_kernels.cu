@@ -175,10 +175,10 @@ __device__ __forceinline__ int operand_of_tile(const FftBatch<OPS>& b, int& tile
 }
 
 template <int N, int T, int OPS>
-__global__ void __launch_bounds__(FBF_COOP_THREADS, 2)
+__global__ void __launch_bounds__(coop_threads(N), coop_blocks(N))
 fft2d_forward_coop_kernel(const __grid_constant__ FftBatch<OPS> b) {
   extern __shared__ __align__(16) char smem[];
-  const int tid = threadIdx.x, nth = blockDim.x;
+  const int tid = threadIdx.x, nth = blockDim.x, lane = tid & 31, warp = tid >> 5;
   const int total = b.tile_end[OPS - 1];
   grid_dependency_wait();
   // persistent blocks: tile w, then w + gridDim.x, ...; the real planes of the next tile are
@@ -202,26 +202,31 @@ fft2d_forward_coop_kernel(const __grid_constant__ FftBatch<OPS> b) {
       for (long long off = (long long)tid * 128; off < plane_bytes; off += (long long)nth * 128) prefetch_l2(src + off);
     }
   }
-  for (int line0 = 0; line0 < g.lines1; line0 += g.chunk) {
-    const int nl = min(g.chunk, g.lines1 - line0);
-    CoopForward<N, T>::row_step1(p, g, smem, tid, nth, row, inner0, line0, nl);
-    __syncthreads();
-    // groups of eight lanes hold the eight residues of one line; mirror residues are
-    // neighbours, so one shuffle hands each lane the partner's odd-indexed outputs
-    constexpr int N1 = CoopForward<N, T>::N1, N2 = CoopForward<N, T>::N2;
-    const int items = nl * N1;
-    for (int base = 0; base < items; base += nth) {
-      float2 u[N2], mirror_odd[N2 / 2];
-      const bool active = CoopForward<N, T>::row_step2_fft(g, smem, base + tid, nl, u);
+  using F = CoopForward<N, T>;
+  constexpr int kTask = F::L::TASK_LINES;
+  {
+    float2 tw[F::N1];  // a lane meets the same n2 in all its items
+    F::row_twiddles(lane, tw);
+    for (int line0 = warp * kTask; line0 < g.lines1; line0 += (nth >> 5) * kTask) {
+      F::row_step1(p, g, smem, lane, row, inner0, line0, tw);
+      __syncwarp();
+      // groups of eight lanes hold the eight residues of one line; mirror residues are
+      // neighbours, so one shuffle hands each lane the partner's odd-indexed outputs
+#pragma unroll 1
+      for (int item = lane; item < kTask * F::N1; item += 32) {
+        float2 u[F::N2], mirror_odd[F::N2 / 2];
+        const bool active = F::row_step2_fft(g, smem, line0, item, u);
 #pragma unroll
-      for (int i = 0; i < N2 / 2; ++i) {
-        mirror_odd[i].x = __shfl_xor_sync(0xffffffffu, u[2 * i + 1].x, 1);
-        mirror_odd[i].y = __shfl_xor_sync(0xffffffffu, u[2 * i + 1].y, 1);
+        for (int i = 0; i < F::N2 / 2; ++i) {  // every lane takes part: the reads above are over after this
+          mirror_odd[i].x = __shfl_xor_sync(0xffffffffu, u[2 * i + 1].x, 1);
+          mirror_odd[i].y = __shfl_xor_sync(0xffffffffu, u[2 * i + 1].y, 1);
+        }
+        __syncwarp();
+        if (active) F::row_step2_split(g, smem, line0, item, u, mirror_odd);
       }
-      if (active) CoopForward<N, T>::row_step2_split(g, smem, base + tid, line0, u, mirror_odd);
     }
-    __syncthreads();
   }
+  __syncthreads();
   CoopForward<N, T>::col_step1(g, smem, tid, nth);
   __syncthreads();
   if (p.spec_bin == 1 && p.spec_inner == (N / 2 + 1) * N)
@@ -233,10 +238,10 @@ fft2d_forward_coop_kernel(const __grid_constant__ FftBatch<OPS> b) {
 }
 
 template <int N, int T, int OPS>
-__global__ void __launch_bounds__(FBF_COOP_THREADS, 2)
+__global__ void __launch_bounds__(coop_threads(N), coop_blocks(N))
 fft2d_inverse_coop_kernel(const __grid_constant__ FftBatch<OPS> b) {
   extern __shared__ __align__(16) char smem[];
-  const int tid = threadIdx.x, nth = blockDim.x;
+  const int tid = threadIdx.x, nth = blockDim.x, lane = tid & 31, warp = tid >> 5;
   const int total = b.tile_end[OPS - 1];
   grid_dependency_wait();
   const int first = (int)blockIdx.x - b.sum_blocks, step = (int)gridDim.x - b.sum_blocks;
@@ -269,13 +274,24 @@ fft2d_inverse_coop_kernel(const __grid_constant__ FftBatch<OPS> b) {
   __syncthreads();
   CoopInverse<N, T>::col_step2(g, smem, tid, nth);
   __syncthreads();
-  for (int line0 = 0; line0 < g.lines1; line0 += g.chunk) {
-    const int nl = min(g.chunk, g.lines1 - line0);
-    CoopInverse<N, T>::row_step1(p, g, smem, tid, nth, line0, nl);
-    __syncthreads();
-    CoopInverse<N, T>::row_step2(p, g, smem, tid, nth, row, inner0, line0, nl);
-    __syncthreads();
+  using I = CoopInverse<N, T>;
+  constexpr int kTask = I::L::TASK_LINES;
+  {
+    float2 tw[I::N1];  // a lane meets the same n2 in all its items
+    I::row_twiddles(lane, tw);
+    for (int line0 = warp * kTask; line0 < g.lines1; line0 += (nth >> 5) * kTask) {
+      float2 v0[I::N1], v1[I::N1];
+      const bool on0 = I::row_step1_fft(p, g, smem, line0, lane, v0);
+      const bool on1 = I::row_step1_fft(p, g, smem, line0, lane + 32, v1);
+      __syncwarp();
+      if (on0) I::row_step1_store(p, g, smem, line0, lane, v0, tw);
+      if (on1) I::row_step1_store(p, g, smem, line0, lane + 32, v1, tw);
+      __syncwarp();
+#pragma unroll 1
+      for (int item = lane; item < kTask * I::N1; item += 32) I::row_step2(p, g, smem, row, inner0, line0, item);
+    }
   }
+  __syncthreads();  // mid is rewritten by the next tile
   }
 }
 
@@ -317,13 +333,9 @@ fft1d_inverse_kernel(const __grid_constant__ FftParams p, const __grid_constant_
   Inverse<N, T>::store(p, g, smem, tid, nth, 0, inner0);
 }
 
-constexpr int kSmemTwoBlocks = 113 * 1024;  // shared memory of one of two resident blocks
-
 // Blocks of a persistent cooperative kernel: as many as are resident at once.
-int persistent_blocks(long long tiles, int smem_bytes) {
-  const int sms = sm_count();
-  const int per_sm = smem_bytes <= kSmemTwoBlocks ? 2 : 1;  // any window at the tile sizes of fft_tile()
-  const long long resident = (long long)sms * per_sm;
+int persistent_blocks(int N, long long tiles) {
+  const long long resident = (long long)sm_count() * coop_blocks(N);
   return (int)(tiles < resident ? tiles : resident);
 }
 
@@ -360,7 +372,8 @@ cudaError_t run_batch(bool inverse, const FftParams* ops, int count, const RowSu
   long long blocks = tiles;
   if constexpr (N > 32) {
     kernel = inverse ? fft2d_inverse_coop_kernel<N, T, OPS> : fft2d_forward_coop_kernel<N, T, OPS>;
-    blocks = persistent_blocks(tiles, smem);
+    static_assert(coop_blocks(N) * (N * CoopLayout<N, T>::PITCH2 * 8 + 1024) <= 228 * 1024, "shared memory of an SM");
+    blocks = persistent_blocks(N, tiles);
   } else {
     if (threads != block_threads<N, T>()) return cudaErrorInvalidConfiguration;
     kernel = inverse ? fft2d_inverse_kernel<N, T, OPS> : fft2d_forward_kernel<N, T, OPS>;

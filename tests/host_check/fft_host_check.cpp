@@ -26,29 +26,29 @@ void run_forward(const FftParams& p) {
       const int inner0 = tile * T;
       std::memset(smem.data(), 0xFF, smem.size());
       if constexpr (N > 32) {
-        for (int line0 = 0; line0 < g.lines1; line0 += g.chunk) {
-          const int nl = std::min(g.chunk, g.lines1 - line0);
-          std::memset(smem.data() + g.off_a, 0xFF, g.off_b - g.off_a);
-          for (int tid = 0; tid < nth; ++tid)
-            CoopForward<N, T>::row_step1(p, g, smem.data(), tid, nth, row, inner0, line0, nl);
-          {  // the device exchanges the transforms of mirror residues by a lane shuffle
-            constexpr int N1 = CoopForward<N, T>::N1, N2 = CoopForward<N, T>::N2;
-            const int items = nl * N1;
-            std::vector<float2> all(static_cast<size_t>(items) * N2);
-            for (int item = 0; item < items; ++item) {
+        using F = CoopForward<N, T>;
+        constexpr int N1 = F::N1, N2 = F::N2, kTask = F::L::TASK_LINES;
+        for (int line0 = 0; line0 < g.lines1; line0 += kTask) {  // a warp's task: 32 lanes, in rounds
+          for (int lane = 0; lane < 32; ++lane) {
+            float2 tw[N1];
+            F::row_twiddles(lane, tw);
+            F::row_step1(p, g, smem.data(), lane, row, inner0, line0, tw);
+          }
+          for (int first = 0; first < kTask * N1; first += 32) {
+            // the device exchanges the transforms of mirror residues by a lane shuffle
+            std::vector<float2> all(static_cast<size_t>(32) * N2, make_float2(NAN, NAN));
+            bool active[32];
+            for (int lane = 0; lane < 32; ++lane) {
               float2 u[N2];
-              CoopForward<N, T>::row_step2_fft(g, smem.data(), item, nl, u);
-              std::copy(u, u + N2, all.begin() + static_cast<size_t>(item) * N2);
+              active[lane] = F::row_step2_fft(g, smem.data(), line0, first + lane, u);
+              if (active[lane]) std::copy(u, u + N2, all.begin() + static_cast<size_t>(lane) * N2);
             }
-            for (int item = 0; item < items; ++item) {
+            for (int lane = 0; lane < 32; ++lane) {
+              if (!active[lane]) continue;
               float2 u[N2], mirror_odd[N2 / 2];
-              std::copy(all.begin() + static_cast<size_t>(item) * N2,
-                        all.begin() + static_cast<size_t>(item + 1) * N2, u);
-              const int partner = item ^ 1;
-              for (int i = 0; i < N2 / 2; ++i)
-                mirror_odd[i] = partner < items ? all[static_cast<size_t>(partner) * N2 + 2 * i + 1]
-                                                : make_float2(NAN, NAN);
-              CoopForward<N, T>::row_step2_split(g, smem.data(), item, line0, u, mirror_odd);
+              std::copy(all.begin() + static_cast<size_t>(lane) * N2, all.begin() + static_cast<size_t>(lane + 1) * N2, u);
+              for (int i = 0; i < N2 / 2; ++i) mirror_odd[i] = all[static_cast<size_t>(lane ^ 1) * N2 + 2 * i + 1];
+              F::row_step2_split(g, smem.data(), line0, first + lane, u, mirror_odd);
             }
           }
         }
@@ -91,13 +91,21 @@ void run_inverse(const FftParams& p, int oh, int ow) {
           else
             CoopInverse<N, T>::template col_step1<false>(p, g, smem.data(), tid, nth, row, inner0);
         for (int tid = 0; tid < nth; ++tid) CoopInverse<N, T>::col_step2(g, smem.data(), tid, nth);
-        for (int line0 = 0; line0 < g.lines1; line0 += g.chunk) {
-          const int nl = std::min(g.chunk, g.lines1 - line0);
-          std::memset(smem.data() + g.off_a, 0xFF, g.off_b - g.off_a);
-          for (int tid = 0; tid < nth; ++tid)
-            CoopInverse<N, T>::row_step1(p, g, smem.data(), tid, nth, line0, nl);
-          for (int tid = 0; tid < nth; ++tid)
-            CoopInverse<N, T>::row_step2(p, g, smem.data(), tid, nth, row, inner0, line0, nl);
+        using I = CoopInverse<N, T>;
+        constexpr int N1 = I::N1, kTask = I::L::TASK_LINES;
+        struct Item {
+          float2 v[N1];
+          bool on;
+        };
+        for (int line0 = 0; line0 < g.lines1; line0 += kTask) {  // a warp's task: 32 lanes, two items each
+          std::vector<Item> items(64);
+          for (int i = 0; i < 64; ++i) items[i].on = I::row_step1_fft(p, g, smem.data(), line0, i, items[i].v);
+          for (int i = 0; i < 64; ++i) {
+            float2 tw[N1];
+            I::row_twiddles(i & 31, tw);
+            if (items[i].on) I::row_step1_store(p, g, smem.data(), line0, i, items[i].v, tw);
+          }
+          for (int i = 0; i < kTask * N1; ++i) I::row_step2(p, g, smem.data(), row, inner0, line0, i);
         }
       } else {
         for (int tid = 0; tid < g.threads; ++tid)

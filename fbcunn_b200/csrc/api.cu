@@ -137,6 +137,7 @@ struct fbfftconv_handle {
   // set by a backward call between its two passes: the second one is handed the gradOutput whose spectrum
   // the first has just left in buf_out
   bool same_grad_output = false;
+  TileViews views;  // where the real tensors of the running pass are tiles of images (TileViewScope)
   char* ws = nullptr;
   bool ws_owned = false;
   // device copies for the host-buffer entry points
@@ -668,9 +669,19 @@ Operand operand(const fbfftconv_handle* h, int stage, const float* real, float2*
                 int cols, int pad_u, int pad_l) {
   return Operand{stage, forward_params(real, spec, d1, d2, rows, cols, pad_u, pad_l, h->plane_major ? 2 : 0, h->N)};
 }
+// The planes of `p` are the tiles of `v`, if that is a view; `by_inner`: the batch is the inner index.
+void apply_view(FftParams& p, const TileView& v, bool by_inner) {
+  if (!v.nw) return;
+  p.view = v;
+  p.view.by_inner = by_inner;
+  p.h = v.th;
+  p.w = pad4(v.tw);
+}
 Operand input_operand(const fbfftconv_handle* h, int stage, const float* input) {
   const fbfftconv_desc& d = h->d;
-  return operand(h, stage, input, h->buf_in(), d.batch, d.n_input_plane, d.input_h, d.input_w, d.pad_h, d.pad_w);
+  Operand op = operand(h, stage, input, h->buf_in(), d.batch, d.n_input_plane, d.input_h, d.input_w, d.pad_h, d.pad_w);
+  apply_view(op.p, h->views.input, false);
+  return op;
 }
 Operand weight_operand(const fbfftconv_handle* h, int stage, const float* weight) {
   const fbfftconv_desc& d = h->d;
@@ -678,7 +689,9 @@ Operand weight_operand(const fbfftconv_handle* h, int stage, const float* weight
 }
 Operand grad_output_operand(const fbfftconv_handle* h, int stage, const float* grad_output) {
   const fbfftconv_desc& d = h->d;
-  return operand(h, stage, grad_output, h->buf_out(), d.batch, d.n_output_plane, h->oH, h->oW, 0, 0);
+  Operand op = operand(h, stage, grad_output, h->buf_out(), d.batch, d.n_output_plane, h->oH, h->oW, 0, 0);
+  apply_view(op.p, h->views.grad_output, false);
+  return op;
 }
 
 // Whether transforms run as one launch.  Up to 32 points always: one wave fewer, and no launch gap.  The
@@ -732,8 +745,12 @@ int contract_grad_input(fbfftconv_handle* h, float2* gi, int* layout, cudaStream
 
 FftParams grad_input_inverse(const fbfftconv_handle* h, const float2* gi, float* grad_input, int layout) {
   const fbfftconv_desc& d = h->d;
-  return inverse_params(gi, grad_input, nullptr, d.batch, d.n_input_plane, d.input_h, d.input_w, d.pad_h, d.pad_w, 0,
-                        layout, h->N);
+  const TileView& v = h->views.grad_input;
+  // of an overlap-save tile the part that no wrapped-around product reaches: from the kernel's extent - 1 on
+  FftParams p = inverse_params(gi, grad_input, nullptr, d.batch, d.n_input_plane, d.input_h, d.input_w,
+                               v.nw ? d.kernel_h - 1 : d.pad_h, v.nw ? d.kernel_w - 1 : d.pad_w, 0, layout, h->N);
+  apply_view(p, v, layout == 1);
+  return p;
 }
 
 // W'^[f][p] = scale/N^2 sum_b conj(O'^[b][f]) I^[b][p] per bin, into the weight buffer.
@@ -760,6 +777,9 @@ RowSum bias_sum(const fbfftconv_handle* h, float* dst, float scale, int accumula
 }
 
 }  // namespace
+
+fbfft::TileViewScope::TileViewScope(fbfftconv_handle* h, const TileViews& views) : h_(h) { h->views = views; }
+fbfft::TileViewScope::~TileViewScope() { h_->views = TileViews{}; }
 
 int fbfftconv_update_output(fbfftconv_handle* h, const float* input, const float* weight,
                             const float* bias, float* output, fbfftconv_stream stream) {
@@ -795,8 +815,9 @@ int fbfftconv_update_output(fbfftconv_handle* h, const float* input, const float
   }
   {
     StageTimer t(h, pass, FBFFTCONV_STAGE_IFFT, s);
-    FBF_TRY(inverse_transform(inverse_params(h->buf_out(), output, bias, B, F, h->oH, h->oW, 0, 0, 0,
-                                             pm ? 2 : (flip ? 1 : 0), h->N), nullptr, h->N, s));
+    FftParams p = inverse_params(h->buf_out(), output, bias, B, F, h->oH, h->oW, 0, 0, 0, pm ? 2 : (flip ? 1 : 0), h->N);
+    apply_view(p, h->views.output, flip);
+    FBF_TRY(inverse_transform(p, nullptr, h->N, s));
   }
   // what the buffers hold now (every pass reads a tensor's spectrum in the one layout it is written in)
   h->have_input_spec = true;

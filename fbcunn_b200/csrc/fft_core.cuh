@@ -314,6 +314,20 @@ static inline FftGeom inverse_geom(int N, int T, int oh, int ow) {
 // ---------------------------------------------------------------------------
 // Kernel parameters
 // ---------------------------------------------------------------------------
+// A real plane that is a tile of a larger image tensor (images, planes, H, W) instead of a plane in memory of
+// its own: element (y, x), y < th, x < tw, of tile (b, ty, tx) is image element (ty*sh + y + oy, tx*sw + x + ox),
+// zero (forward) or not stored (inverse) outside the image.  FftParams::h is th and FftParams::w is tw rounded
+// up to a multiple of four: rows are staged on 16-byte boundaries, the columns beyond tw as zeros.
+struct TileView {
+  int nh, nw;          // tiles per image; nw = 0: no view, planes lie in memory one after the other
+  int th, tw;
+  int sh, sw;          // step between the origins of neighbouring tiles
+  int oy, ox;          // image coordinate of the first element of tile (0, 0)
+  int H, W;            // extent of the image
+  int planes;          // planes of an image
+  int by_inner;        // the tile number (b*nh + ty)*nw + tx is the inner index and the plane the row index
+};
+
 // A tile is T planes with consecutive `inner` index at one `row` of the spectrum.
 // Real plane of (row, inner) starts at real + (row*real_row_stride +
 // inner*real_inner_stride) * h * w  (strides counted in planes), so the same
@@ -333,7 +347,26 @@ struct FftParams {
   int kc;                 // padded inner extent of the spectrum (multiple of 4)
   long long real_row_stride, real_inner_stride;
   int accumulate;         // inverse only: real_out += result
+  TileView view;          // thread-per-line sizes of 8 points and more
 };
+
+// Place of one tile of a view: offset of its image plane, image coordinates of its first element.
+struct TilePlace {
+  long long plane;
+  int y0, x0;
+};
+FBF_HD TilePlace tile_place(const TileView& v, int row, int inner) {
+  const int tile = v.by_inner ? inner : row, plane = v.by_inner ? row : inner;
+  const int tx = tile % v.nw, rest = tile / v.nw;
+  const int ty = rest % v.nh, b = rest / v.nh;
+  TilePlace r;
+  r.plane = ((long long)b * v.planes + plane) * ((long long)v.H * v.W);
+  r.y0 = ty * v.sh + v.oy;
+  r.x0 = tx * v.sw + v.ox;
+  return r;
+}
+// log2 of the lanes that copy the rows of a tile w columns wide together.
+FBF_HD int tile_group_shift(int w) { return w <= 8 ? 3 : w <= 16 ? 4 : 5; }
 
 // Registers a thread keeps across a barrier (thread-per-line sizes only).
 template <int N>
@@ -372,9 +405,38 @@ struct Forward {
     return p.real_in + (row * p.real_row_stride + inner * p.real_inner_stride) * ((long long)p.h * p.w);
   }
 
+  // Phase 0 where the planes are tiles of images: a group of lanes takes a plane, a lane a column of it.
+  static FBF_HD void load_tiles(const FftParams& p, const FftGeom& g, char* smem, int tid, int nthreads, int row,
+                                int inner0) {
+    float* stage = reinterpret_cast<float*>(smem + g.off_a);
+    const TileView& v = p.view;
+    const int shift = tile_group_shift(p.w);
+    const int x = tid & ((1 << shift) - 1);
+    for (int t = tid >> shift; t < T; t += nthreads >> shift) {
+      if (inner0 + t >= p.n_inner) break;
+      const TilePlace at = tile_place(v, row, inner0 + t);
+      const float* src = p.real_in + at.plane + (long long)at.y0 * v.W + (at.x0 + x);
+      float* dst = stage + t * g.pitch1 + x;
+      const bool in = x < v.tw && (unsigned)(at.x0 + x) < (unsigned)v.W;
+      if (x < p.w) {
+#pragma unroll 4
+        for (int y = 0; y < p.h; ++y) {
+          if (in && (unsigned)(at.y0 + y) < (unsigned)v.H)
+            async_copy4(dst + y * p.w, src + (long long)y * v.W);
+          else
+            dst[y * p.w] = 0.f;
+        }
+      }
+    }
+    async_copy_wait();
+  }
+
   // Phase 0: real planes -> stage, plane t at stage + t*pitch1 + phase16(plane); warps take planes.
+  // VIEW (here and below): the planes may be tiles of images, staged without a shift.
+  template <bool VIEW = false>
   static FBF_HD void load(const FftParams& p, const FftGeom& g, char* smem, int tid, int nthreads,
                           int row, int inner0) {
+    if (VIEW && p.view.nw) return load_tiles(p, g, smem, tid, nthreads, row, inner0);
     float* stage = reinterpret_cast<float*>(smem + g.off_a);
     const int hw = p.h * p.w;
     // small planes: a warp splits into groups of 8 or 16 lanes that take one plane each
@@ -398,13 +460,14 @@ struct Forward {
   }
 
   // Phase 1a: rows (j, j+hh) of plane t into registers as (re, im), zero outside the plane.
+  template <bool VIEW = false>
   static FBF_HD void row_fetch(const FftParams& p, const FftGeom& g, const char* smem, int line, int row,
                                int inner0, LineRegs<N>& regs) {
     if (line >= g.lines1) return;
     const float* stage = reinterpret_cast<const float*>(smem + g.off_a);
     const int j = line / T, t = line - j * T;
     const bool live = inner0 + t < p.n_inner;
-    const float* sp = stage + t * g.pitch1 + phase16(plane_ptr(p, row, inner0 + t));
+    const float* sp = stage + t * g.pitch1 + (VIEW && p.view.nw ? 0 : phase16(plane_ptr(p, row, inner0 + t)));
     const int ya = j - p.off_y, yb = ya + g.hh;
     const bool va = live && (unsigned)ya < (unsigned)p.h, vb = live && (unsigned)yb < (unsigned)p.h;
     const float* pa = sp + ya * p.w - p.off_x;
@@ -523,13 +586,14 @@ struct Inverse {
 
   // Phase 2b: inverse transform along x, stage the crop columns as real rows, plane t at
   // stage + t*pitch1 + phase16(its destination).
+  template <bool VIEW = false>
   static FBF_HD void row_pass(const FftParams& p, const FftGeom& g, char* smem, int line, int row,
                               int inner0, LineRegs<N>& regs) {
     if (line >= g.lines1) return;
     float* stage = reinterpret_cast<float*>(smem + g.off_a);
     const int j = line / T, t = line - j * T;
     const bool has_b = (j + g.hh) < g.he;
-    const int shift = phase16(plane_ptr(p, g, row, inner0 + t));
+    const int shift = VIEW && p.view.nw ? 0 : phase16(plane_ptr(p, g, row, inner0 + t));
     float* sa = stage + t * g.pitch1 + shift + j * g.we - p.off_x;
     float* sb = sa + g.hh * g.we;
     const unsigned we = (unsigned)g.we;
@@ -564,9 +628,35 @@ struct Inverse {
     return p.accumulate ? *dst + (v + bias) : v + bias;
   }
 
+  // Phase 3 where the planes are tiles of images: the part inside the image is stored.
+  static FBF_HD void store_tiles(const FftParams& p, const FftGeom& g, const char* smem, int tid, int nthreads,
+                                 int row, int inner0) {
+    const float* stage = reinterpret_cast<const float*>(smem + g.off_a);
+    const TileView& v = p.view;
+    const int shift = tile_group_shift(g.we);
+    const int x = tid & ((1 << shift) - 1);
+    for (int t = tid >> shift; t < T; t += nthreads >> shift) {
+      const int inner = inner0 + t;
+      if (inner >= p.n_inner) break;
+      const float bias = p.bias ? p.bias[p.bias_by_row ? row : inner] : 0.f;
+      const TilePlace at = tile_place(v, row, inner);
+      float* dst = p.real_out + at.plane + (long long)at.y0 * v.W + (at.x0 + x);
+      const float* src = stage + t * g.pitch1 + x;
+      if (x >= v.tw || (unsigned)(at.x0 + x) >= (unsigned)v.W) continue;
+#pragma unroll 4
+      for (int y = 0; y < g.he; ++y)
+        if ((unsigned)(at.y0 + y) < (unsigned)v.H) {
+          float* d = dst + (long long)y * v.W;
+          *d = finish(p, src[y * g.we], bias, d);
+        }
+    }
+  }
+
   // Phase 3: staged planes -> global in 16-byte pieces, bias added per plane; warps take planes.
+  template <bool VIEW = false>
   static FBF_HD void store(const FftParams& p, const FftGeom& g, const char* smem, int tid,
                            int nthreads, int row, int inner0) {
+    if (VIEW && p.view.nw) return store_tiles(p, g, smem, tid, nthreads, row, inner0);
     const float* stage = reinterpret_cast<const float*>(smem + g.off_a);
     const int per_plane = g.he * g.we;
     const int lp_shift = copy_group_shift(per_plane);

@@ -110,7 +110,8 @@ __device__ __forceinline__ void with_operand(const FftBatch<OPS>& b, int tile, B
   }
 }
 
-template <int N, int T, int OPS>
+// VIEW: planes of some operand are tiles of images (a kernel of its own, so that the others stay as they are).
+template <int N, int T, int OPS, bool VIEW>
 __global__ void __launch_bounds__(block_threads<N, T>())
 fft2d_forward_kernel(const __grid_constant__ FftBatch<OPS> b) {
   extern __shared__ __align__(16) char smem[];
@@ -119,10 +120,10 @@ fft2d_forward_kernel(const __grid_constant__ FftBatch<OPS> b) {
   with_operand(b, blockIdx.x, [&](const FftParams& p, const FftGeom& g, int tile, int tiles_x) {
     const int row = tile / tiles_x;
     const int inner0 = (tile - row * tiles_x) * T;
-    Forward<N, T>::load(p, g, smem, tid, blockDim.x, row, inner0);
+    Forward<N, T>::template load<VIEW>(p, g, smem, tid, blockDim.x, row, inner0);
     __syncthreads();
     LineRegs<N> regs;
-    Forward<N, T>::row_fetch(p, g, smem, tid, row, inner0, regs);
+    Forward<N, T>::template row_fetch<VIEW>(p, g, smem, tid, row, inner0, regs);
     __syncthreads();  // the column buffer aliases the staged planes
     Forward<N, T>::row_pass(g, smem, tid, regs);
     __syncthreads();
@@ -130,7 +131,7 @@ fft2d_forward_kernel(const __grid_constant__ FftBatch<OPS> b) {
   });
 }
 
-template <int N, int T, int OPS>
+template <int N, int T, int OPS, bool VIEW>
 __global__ void __launch_bounds__(block_threads<N, T>())
 fft2d_inverse_kernel(const __grid_constant__ FftBatch<OPS> b) {
   extern __shared__ __align__(16) char smem[];
@@ -148,9 +149,9 @@ fft2d_inverse_kernel(const __grid_constant__ FftBatch<OPS> b) {
     LineRegs<N> regs;
     Inverse<N, T>::row_fetch(g, smem, tid, regs);
     __syncthreads();  // the staged output aliases the column buffer
-    Inverse<N, T>::row_pass(p, g, smem, tid, row, inner0, regs);
+    Inverse<N, T>::template row_pass<VIEW>(p, g, smem, tid, row, inner0, regs);
     __syncthreads();
-    Inverse<N, T>::store(p, g, smem, tid, blockDim.x, row, inner0);
+    Inverse<N, T>::template store<VIEW>(p, g, smem, tid, blockDim.x, row, inner0);
   });
 }
 
@@ -351,9 +352,11 @@ cudaError_t run_batch(bool inverse, const FftParams* ops, int count, const RowSu
   FftBatch<OPS> b{};
   long long tiles = 0;
   int smem = 0;
+  bool view = false;
   for (int i = 0; i < OPS; ++i) {
     if (i < count) {
       b.p[i] = ops[i];
+      view |= ops[i].view.nw != 0;
       b.g[i] = inverse ? inverse_geom(N, T, ops[i].h, ops[i].w)
                        : forward_geom(N, T, ops[i].h, ops[i].w, ops[i].off_y, ops[i].off_x);
       b.tiles_x[i] = ((inverse ? ops[i].n_inner : ops[i].kc) + T - 1) / T;
@@ -376,8 +379,11 @@ cudaError_t run_batch(bool inverse, const FftParams* ops, int count, const RowSu
     blocks = persistent_blocks(N, tiles);
   } else {
     if (threads != block_threads<N, T>()) return cudaErrorInvalidConfiguration;
-    kernel = inverse ? fft2d_inverse_kernel<N, T, OPS> : fft2d_forward_kernel<N, T, OPS>;
+    kernel = inverse ? fft2d_inverse_kernel<N, T, OPS, false> : fft2d_forward_kernel<N, T, OPS, false>;
+    if constexpr (N >= 8)
+      if (view) kernel = inverse ? fft2d_inverse_kernel<N, T, OPS, true> : fft2d_forward_kernel<N, T, OPS, true>;
   }
+  if (view && !tile_view_supported(N)) return cudaErrorInvalidConfiguration;
   cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
   if (e != cudaSuccess) return e;
   e = launch_dependent(kernel, dim3((unsigned)(blocks + b.sum_blocks)), threads, smem, stream, b);

@@ -5,6 +5,8 @@
 
 #include "fft_core.cuh"
 
+struct fbfftconv_handle;
+
 namespace fbfft {
 
 // Counts every kernel this library launches (reported through the C ABI).
@@ -61,6 +63,8 @@ struct RowSum {
 };
 
 constexpr int kMaxFftOps = 3;
+// Transform sizes whose kernels take tiles of images as planes (FftParams::view).
+constexpr bool tile_view_supported(int N) { return N >= 8 && N <= 32; }
 // Transforms of up to kMaxFftOps operands in one launch (all of the same size N).
 cudaError_t launch_forward(const FftParams* ops, int count, int N, cudaStream_t stream);
 cudaError_t launch_inverse(const FftParams* ops, int count, const RowSum* sum, int N, cudaStream_t stream);
@@ -137,6 +141,22 @@ int peer_error(bool reset);
 // Makes one bounded wait on a peer flag run out on purpose: 1 = it gave up (code 1 left for
 // peer_error), 0 = it did not, < 0 = CUDA error.
 int peer_wait_probe(cudaStream_t stream);
+
+// Makes the passes of `h` read and write tiles of image tensors instead of planes of their own, for as long as
+// the object lives: `input` and `grad_output` where they are transformed, `output` and `grad_input` where they
+// are stored (without their views: contiguous planes).  grad_input's tiles are then disjoint and complete
+// (overlap-save), which takes gradOutput tiles that overlap, with the kernel's reach before them.
+struct TileViews {
+  TileView input{}, output{}, grad_output{}, grad_input{};
+};
+class TileViewScope {
+ public:
+  TileViewScope(fbfftconv_handle* h, const TileViews& views);
+  ~TileViewScope();
+
+ private:
+  fbfftconv_handle* h_;
+};
 
 // Records `message` as the calling thread's last error (what fbfftconv_last_error
 // returns) and hands `code` back, for entry points that live outside api.cu.

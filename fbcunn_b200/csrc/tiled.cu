@@ -8,11 +8,17 @@
 //
 // The tiles of one image are extra batch entries of one untiled pass:
 //     updateOutput        input tiles (overlapping)   -> output tiles (disjoint)
-//     updateGradInput     gradOutput tiles (disjoint) -> gradInput tiles, overlap-added
+//     updateGradInput     gradOutput tiles (overlapping) -> gradInput tiles (disjoint), or
+//                         gradOutput tiles (disjoint) -> gradInput tiles, overlap-added
 //     accGradParameters   the contraction's sum over the batch is also the sum over tiles
-// Cutting, assembling and the overlap-add are the three small kernels below (each element
-// is gathered, so the result does not depend on timing); the tile buffers belong to the
-// tiled handle.
+// Up to 32 points the transforms read the tiles out of the image tensors and store them there themselves
+// (TileView): an image then crosses memory once per pass instead of three times.  gradInput is made of disjoint
+// tiles by overlap-save as well, from gradOutput tiles of the full tile size, so that nothing is added up; only
+// where accGradParameters takes over the gradOutput spectrum (which must be that of the disjoint tiles), or the
+// output's tiles do not cover the input, is it overlap-added from a tile buffer.  The 64- and 128-point
+// transforms take tiles that the kernels below cut, assemble and overlap-add (each element is gathered, so the
+// result does not depend on timing).  32 x 64 x 224 x 224, 64 filters 3 x 3, 32-pixel tiles, three passes:
+// cutting, assembling and adding up in kernels of their own 4850 us, this 2780.
 #include <cstdio>
 
 #include "../../include/fbfftconv.h"
@@ -115,8 +121,10 @@ struct fbfftconv_tiled {
   int device;
   int oH, oW;              // output extent of the layer
   int th, tw, sh, sw, nh, nw;
+  bool views;              // the transforms work on the image tensors themselves
+  bool save_grad_input;    // (views) gradInput by overlap-save
   float* in_tiles = nullptr;   // (B*nh*nw, P, th, tw): input tiles / gradInput tiles
-  float* out_tiles = nullptr;  // (B*nh*nw, F, sh, sw): output tiles / gradOutput tiles
+  float* out_tiles = nullptr;  // (B*nh*nw, F, sh, sw): output tiles / gradOutput tiles; none with views
 };
 
 namespace {
@@ -128,6 +136,37 @@ TileGeom input_geom(const fbfftconv_tiled* t) {
 TileGeom output_geom(const fbfftconv_tiled* t) {
   const fbfftconv_desc& d = t->d;
   return TileGeom{d.batch, d.n_output_plane, t->oH, t->oW, t->sh, t->sw, t->sh, t->sw, t->nh, t->nw, 0, 0};
+}
+
+// floats of the two tile buffers
+size_t in_tile_floats(const fbfftconv_tiled* t) {
+  return t->views && t->save_grad_input ? 0 : (size_t)t->d.batch * t->nh * t->nw * t->d.n_input_plane * t->th * t->tw;
+}
+size_t out_tile_floats(const fbfftconv_tiled* t) {
+  return t->views ? 0 : (size_t)t->d.batch * t->nh * t->nw * t->d.n_output_plane * t->sh * t->sw;
+}
+
+TileView view_of(const TileGeom& g) {
+  return TileView{g.nh, g.nw, g.th, g.tw, g.sh, g.sw, g.oy, g.ox, g.H, g.W, g.C, 0};
+}
+TileView input_view(const fbfftconv_tiled* t) { return view_of(input_geom(t)); }
+TileView output_view(const fbfftconv_tiled* t) { return view_of(output_geom(t)); }
+// gradInput element Y sums gradOutput elements Y + pad - k, k < kernel: a tile of sh gradInput rows from row
+// Y0 on needs the th = sh + kernel - 1 gradOutput rows from Y0 + pad - (kernel - 1) on.
+TileView grad_output_save_view(const fbfftconv_tiled* t) {
+  TileView v = output_view(t);
+  v.th = t->th;
+  v.tw = t->tw;
+  v.oy = t->d.pad_h - t->d.kernel_h + 1;
+  v.ox = t->d.pad_w - t->d.kernel_w + 1;
+  return v;
+}
+TileView grad_input_save_view(const fbfftconv_tiled* t) {
+  TileView v = input_view(t);
+  v.th = t->sh;
+  v.tw = t->sw;
+  v.oy = v.ox = 0;
+  return v;
 }
 
 int tiled_fail(int code, const char* message) { return report_error(code, message); }
@@ -145,8 +184,8 @@ struct Guard {
 
 int ensure_tiles(fbfftconv_tiled* t) {
   if (t->in_tiles) return FBFFTCONV_OK;
-  const size_t tiles = (size_t)t->d.batch * t->nh * t->nw;
-  const size_t n_in = tiles * t->d.n_input_plane * t->th * t->tw, n_out = tiles * t->d.n_output_plane * t->sh * t->sw;
+  const size_t n_in = in_tile_floats(t), n_out = out_tile_floats(t);
+  if (n_in + n_out == 0) return FBFFTCONV_OK;
   void* p = nullptr;
   cudaError_t e = cudaMalloc(&p, (n_in + n_out) * sizeof(float));
   if (e != cudaSuccess) {
@@ -215,6 +254,9 @@ int fbfftconv_tiled_create(const fbfftconv_desc* desc, int tile_h, int tile_w, f
     delete t;
     return rc;
   }
+  t->views = tile_view_supported(fbfftconv_fft_size(t->inner));
+  t->save_grad_input = !(d.flags & FBFFTCONV_REUSE_OUTPUT) && ceil_div(d.input_h, t->sh) <= t->nh &&
+                       ceil_div(d.input_w, t->sw) <= t->nw;
   t->device = d.device;
   if (t->device < 0 && cudaGetDevice(&t->device) != cudaSuccess) {
     cudaGetLastError();
@@ -239,9 +281,7 @@ fbfftconv_handle* fbfftconv_tiled_inner(fbfftconv_tiled* t) { return t ? t->inne
 
 size_t fbfftconv_tiled_workspace_bytes(const fbfftconv_tiled* t) {
   if (!t) return 0;
-  const size_t tiles = (size_t)t->d.batch * t->nh * t->nw;
-  return fbfftconv_workspace_bytes(t->inner) +
-         tiles * ((size_t)t->d.n_input_plane * t->th * t->tw + (size_t)t->d.n_output_plane * t->sh * t->sw) * sizeof(float);
+  return fbfftconv_workspace_bytes(t->inner) + (in_tile_floats(t) + out_tile_floats(t)) * sizeof(float);
 }
 
 int fbfftconv_tiled_geometry(const fbfftconv_tiled* t, int32_t out[6]) {
@@ -264,6 +304,13 @@ int fbfftconv_tiled_update_output(fbfftconv_tiled* t, const float* input, const 
   TILED_TRY(validate_device_pointer(t->device, output, "output"));
   TILED_TRY(ensure_tiles(t));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (t->views) {
+    TileViews v;
+    v.input = input_view(t);
+    v.output = output_view(t);
+    TileViewScope scope(t->inner, v);
+    return fbfftconv_update_output(t->inner, input, weight, bias, output, stream);
+  }
   TILED_CUDA(launch_cut(input, t->in_tiles, input_geom(t), s));
   TILED_TRY(fbfftconv_update_output(t->inner, t->in_tiles, weight, nullptr, t->out_tiles, stream));
   // the bias goes on once, while the tiles are put together (fbcunn/SpatialConvolutionFFTTiled.lua:541-544)
@@ -279,8 +326,18 @@ int fbfftconv_tiled_update_grad_input(fbfftconv_tiled* t, const float* grad_outp
   TILED_TRY(validate_device_pointer(t->device, grad_input, "gradInput"));
   TILED_TRY(ensure_tiles(t));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  TILED_CUDA(launch_cut(grad_output, t->out_tiles, output_geom(t), s));
-  TILED_TRY(fbfftconv_update_grad_input(t->inner, t->out_tiles, weight, t->in_tiles, stream));
+  if (t->views) {
+    TileViews v;
+    v.grad_output = t->save_grad_input ? grad_output_save_view(t) : output_view(t);
+    if (t->save_grad_input) v.grad_input = grad_input_save_view(t);
+    TileViewScope scope(t->inner, v);
+    TILED_TRY(fbfftconv_update_grad_input(t->inner, grad_output, weight,
+                                          t->save_grad_input ? grad_input : t->in_tiles, stream));
+    if (t->save_grad_input) return FBFFTCONV_OK;
+  } else {
+    TILED_CUDA(launch_cut(grad_output, t->out_tiles, output_geom(t), s));
+    TILED_TRY(fbfftconv_update_grad_input(t->inner, t->out_tiles, weight, t->in_tiles, stream));
+  }
   TILED_CUDA(launch_gather(t->in_tiles, grad_input, nullptr, input_geom(t), s));  // overlap-add
   return FBFFTCONV_OK;
 }
@@ -293,6 +350,13 @@ int fbfftconv_tiled_acc_grad_parameters(fbfftconv_tiled* t, const float* input, 
   TILED_TRY(validate_device_pointer(t->device, grad_output, "gradOutput"));
   TILED_TRY(ensure_tiles(t));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (t->views) {
+    TileViews v;
+    v.input = input_view(t);
+    v.grad_output = output_view(t);
+    TileViewScope scope(t->inner, v);
+    return fbfftconv_acc_grad_parameters(t->inner, input, grad_output, grad_weight, grad_bias, scale, stream);
+  }
   TILED_CUDA(launch_cut(input, t->in_tiles, input_geom(t), s));
   TILED_CUDA(launch_cut(grad_output, t->out_tiles, output_geom(t), s));
   return fbfftconv_acc_grad_parameters(t->inner, t->in_tiles, t->out_tiles, grad_weight, grad_bias, scale, stream);

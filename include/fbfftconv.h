@@ -153,14 +153,16 @@ int fbfftconv_backward(fbfftconv_handle* h, const float* input, const float* gra
  * must not exceed 65535); cutting, assembling (with the bias, added once) and the overlap-add of
  * updateGradInput are kernels of the library, and accGradParameters' sum over the batch is also the
  * sum over tiles.  desc describes the whole layer (its flags apply to the untiled layer of the
- * tiles); tile_h / tile_w are clipped to the padded image.  The tile buffers are allocated with
- * cudaMalloc at the first pass.  fbfftconv_tiled_inner gives the untiled layer's handle (owned by the
+ * tiles); tile_h / tile_w are clipped to the padded image.  Transforms of up to 32 points read
+ * and store the tiles in the caller's tensors; where tile buffers are needed (larger transforms, gradInput
+ * with FBFFTCONV_REUSE_OUTPUT or beyond the output's tiles) they are allocated with cudaMalloc at the first
+ * pass.  fbfftconv_tiled_inner gives the untiled layer's handle (owned by the
  * tiled one) for fbfftconv_comm_init, the profile and status queries. */
 typedef struct fbfftconv_tiled fbfftconv_tiled;
 int fbfftconv_tiled_create(const fbfftconv_desc* desc, int tile_h, int tile_w, fbfftconv_tiled** out);
 int fbfftconv_tiled_destroy(fbfftconv_tiled* t);
 fbfftconv_handle* fbfftconv_tiled_inner(fbfftconv_tiled* t);
-/* Device bytes the tiled passes need: the untiled layer's scratch plus the two tile buffers. */
+/* Device bytes the tiled passes need: the untiled layer's scratch plus the tile buffers, if any. */
 size_t fbfftconv_tiled_workspace_bytes(const fbfftconv_tiled* t);
 /* out = { input tile h, w; output tile (= step of the input tiles) h, w; tiles per image along h, w }
  * (the geometry of fbcunn/SpatialConvolutionFFTTiled.lua:55-221 for disjoint output tiles). */

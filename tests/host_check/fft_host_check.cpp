@@ -60,9 +60,9 @@ void run_forward(const FftParams& p) {
             CoopForward<N, T>::template col_step2<false>(p, g, smem.data(), tid, nth, row, inner0);
       } else {
         for (int tid = 0; tid < g.threads; ++tid)
-          Forward<N, T>::load(p, g, smem.data(), tid, g.threads, row, inner0);
+          Forward<N, T>::template load<true>(p, g, smem.data(), tid, g.threads, row, inner0);
         for (int tid = 0; tid < g.threads; ++tid)
-          Forward<N, T>::row_fetch(p, g, smem.data(), tid, row, inner0, regs[tid]);
+          Forward<N, T>::template row_fetch<true>(p, g, smem.data(), tid, row, inner0, regs[tid]);
         std::memset(smem.data(), 0xFF, smem.size());  // aliasing: the row buffer is dead now
         for (int tid = 0; tid < g.threads; ++tid)
           Forward<N, T>::row_pass(g, smem.data(), tid, regs[tid]);
@@ -114,9 +114,9 @@ void run_inverse(const FftParams& p, int oh, int ow) {
           Inverse<N, T>::row_fetch(g, smem.data(), tid, regs[tid]);
         std::memset(smem.data() + g.off_b, 0xFF, smem.size() - g.off_b);  // mid is dead now
         for (int tid = 0; tid < g.threads; ++tid)
-          Inverse<N, T>::row_pass(p, g, smem.data(), tid, row, inner0, regs[tid]);
+          Inverse<N, T>::template row_pass<true>(p, g, smem.data(), tid, row, inner0, regs[tid]);
         for (int tid = 0; tid < g.threads; ++tid)
-          Inverse<N, T>::store(p, g, smem.data(), tid, g.threads, row, inner0);
+          Inverse<N, T>::template store<true>(p, g, smem.data(), tid, g.threads, row, inner0);
       }
     }
   }
@@ -253,6 +253,26 @@ int hostcheck_fft_inverse(const float* spec, float* real, const float* bias, int
   p.real_row_stride = row_stride; p.real_inner_stride = inner_stride;
   p.accumulate = accumulate;
   return dispatch(true, p, N, T, oh, ow);
+}
+
+// The planes are the tiles of images (B, planes, H, W): v = {nh, nw, th, tw, sh, sw, oy, ox, H, W, by_inner}.
+int hostcheck_fft_tiles(int inverse, float* images, float* spec, const float* bias, int N, int T, const int* v,
+                        int B, int planes, int kc, int off_y, int off_x) {
+  FftParams p{};
+  p.view = TileView{v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7], v[8], v[9], planes, v[10]};
+  p.real_in = images;
+  p.real_out = images;
+  p.spec = reinterpret_cast<float2*>(spec);
+  p.bias = bias;
+  p.bias_by_row = v[10];
+  p.h = v[2]; p.w = (v[3] + 3) / 4 * 4;
+  p.off_y = off_y; p.off_x = off_x;
+  const int tiles = B * v[0] * v[1];
+  p.n_rows = v[10] ? planes : tiles;
+  p.n_inner = v[10] ? tiles : planes;
+  p.kc = kc;
+  set_layout(p, N, 0);
+  return dispatch(inverse != 0, p, N, T, p.h, p.w);
 }
 
 int hostcheck_forward_smem_bytes(int N, int T, int h, int w, int pad_u, int pad_l) {

@@ -146,3 +146,59 @@ def test_1d_transforms(hc, N, T):
                                   N, T, h, n, off, planes) == 0
         ref_t = N * full[:, off:off + n]
         assert np.abs(out - ref_t).max() <= 3e-6 * np.abs(ref_t).max() * N
+
+
+# image extent, padding and kernel per tile size: ragged last tiles, tiles that hang over on every side, one tile
+TILES = [(8, 19, 21, 2, 1, 3, 2), (16, 70, 61, 2, 1, 5, 4), (32, 70, 61, 0, 3, 3, 7), (32, 20, 31, 1, 1, 3, 3)]
+
+
+@pytest.mark.parametrize("by_inner", (0, 1))
+@pytest.mark.parametrize("tile,H,W,pU,pL,kH,kW", TILES)
+def test_tiles_of_images(hc, tile, H, W, pU, pL, kH, kW, by_inner):
+    """Planes that are tiles of images: the forward transform against the DFT of the tiles cut out here, the
+    inverse against the transform of contiguous planes, put together here."""
+    N, T = tile, (16 if tile <= 16 else 8)
+    B, C = 2, 5
+    rng = np.random.default_rng(tile + W)
+    th, tw = min(tile, H + 2 * pU), min(tile, W + 2 * pL)
+    sh, sw = th - kH + 1, tw - kW + 1
+    nh, nw = -(-(H + 2 * pU - kH + 1) // sh), -(-(W + 2 * pL - kW + 1) // sw)
+    tiles, half = B * nh * nw, N // 2 + 1
+    inner = tiles if by_inner else C
+    kc = (inner + 3) // 4 * 4
+
+    def run(inverse, images, spec, bias, th, tw, oy, ox, off_y, off_x):
+        v = (ctypes.c_int * 11)(nh, nw, th, tw, sh, sw, oy, ox, H, W, by_inner)
+        assert hc.hostcheck_fft_tiles(inverse, images.ctypes.data_as(ctypes.c_void_p),
+                                      spec.ctypes.data_as(ctypes.c_void_p),
+                                      bias.ctypes.data_as(ctypes.c_void_p) if bias is not None else None,
+                                      N, T, v, B, C, kc, off_y, off_x) == 0
+
+    images = rng.standard_normal((B, C, H, W)).astype(np.float32)
+    padded = np.zeros((B, C, nh * sh + tile + pU, nw * sw + tile + pL), np.float32)
+    padded[:, :, pU:pU + H, pL:pL + W] = images
+    cut = np.stack([padded[b, :, y * sh:y * sh + th, x * sw:x * sw + tw]
+                    for b in range(B) for y in range(nh) for x in range(nw)])
+    if by_inner:
+        cut = cut.transpose(1, 0, 2, 3)
+    spec = np.full((half * N, cut.shape[0], kc, 2), np.nan, np.float32)
+    run(0, images, spec, None, th, tw, -pU, -pL, 0, 0)
+    ref = _bin_major(spectral.rfft2_padded(np.ascontiguousarray(cut), N, N, 0, 0))
+    got = spec[:, :, :inner, 0] + 1j * spec[:, :, :inner, 1]
+    assert np.abs(got - ref).max() <= 5e-6 * np.abs(ref).max()
+    # inverse: the disjoint part of every tile, from (kH - 1, kW - 1) on
+    planes = np.full((cut.shape[0], inner, sh, sw), np.nan, np.float32)
+    assert hc.hostcheck_fft_inverse(spec.ctypes.data_as(ctypes.c_void_p), planes.ctypes.data_as(ctypes.c_void_p),
+                                    None, N, T, sh, sw, kH - 1, kW - 1, cut.shape[0], inner, kc,
+                                    LL(inner), LL(1), 0, 0) == 0
+    bias = rng.standard_normal(C).astype(np.float32)
+    whole = np.full((B, C, nh * sh, nw * sw), np.nan, np.float32)
+    flat = planes.transpose(1, 0, 2, 3) if by_inner else planes
+    for i in range(tiles):
+        b, y, x = i // (nh * nw), i // nw % nh, i % nw
+        whole[b, :, y * sh:(y + 1) * sh, x * sw:(x + 1) * sw] = flat[i] + bias[:, None, None]
+    out = np.full((B, C, H, W), np.nan, np.float32)
+    run(1, out, spec, bias, sh, sw, 0, 0, kH - 1, kW - 1)
+    h, w = min(H, nh * sh), min(W, nw * sw)
+    assert np.array_equal(out[:, :, :h, :w], whole[:, :, :h, :w])
+    assert np.isnan(out[:, :, h:]).all() and np.isnan(out[:, :, :, w:]).all()

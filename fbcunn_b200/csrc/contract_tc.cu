@@ -116,15 +116,31 @@ __device__ __forceinline__ void tmem_alloc(uint32_t* smem_result, uint32_t colum
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t columns) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(columns) : "memory");
 }
-__device__ __forceinline__ void umma_tf32(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+// A tile in tensor memory (row m in lane m, one TF32 value of K per column), B in shared memory.
+__device__ __forceinline__ void umma_tf32(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
                                           uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
       : "memory");
 }
+// 8 or 16 columns of this warp's 32 lanes (a lane of the warp = a lane of tensor memory).
+__device__ __forceinline__ void tmem_store_cols(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+               ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
+__device__ __forceinline__ void tmem_store_cols(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_store_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                : "memory");
@@ -216,16 +232,19 @@ EncodeTiledFn encode_fn() {
 }
 
 // [bins][rows][inner_floats] fp32, box {box_floats, box_rows, 1}; out-of-range elements read as zero.
+// swizzle: the box's rows, 64 or 128 bytes long, land with the swizzle of that span.
 bool make_map(CUtensorMap* map, const void* base, int inner_floats, int rows, int bins, int box_rows,
-              int box_floats) {
+              int box_floats, bool swizzle) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return false;
   const cuuint64_t dims[3] = {(cuuint64_t)inner_floats, (cuuint64_t)rows, (cuuint64_t)bins};
   const cuuint64_t strides[2] = {(cuuint64_t)inner_floats * 4, (cuuint64_t)inner_floats * 4 * (cuuint64_t)rows};
   const cuuint32_t box[3] = {(cuuint32_t)box_floats, (cuuint32_t)box_rows, 1};
   const cuuint32_t elem[3] = {1, 1, 1};
+  const CUtensorMapSwizzle mode = !swizzle ? CU_TENSOR_MAP_SWIZZLE_NONE
+                                  : box_floats == 16 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B;
   return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(base), dims, strides, box, elem,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, mode, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -245,16 +264,19 @@ namespace {
 struct MapKey {
   const void* base;
   int inner_floats, rows, bins, box_rows, box_floats;
+  bool swizzle;
   bool operator==(const MapKey& o) const {
     return base == o.base && inner_floats == o.inner_floats && rows == o.rows && bins == o.bins &&
-           box_rows == o.box_rows && box_floats == o.box_floats;
+           box_rows == o.box_rows && box_floats == o.box_floats &&
+           swizzle == o.swizzle;
   }
 };
 // Map of one operand with `rows` rows of the tile dimension (tile of `tile_rows`) and depth k:
 // stored [bins][rows][ld] (ld >= k) or, transposed, [bins][k][ld] (ld >= rows).
-MapKey operand_key(const void* base, int rows, int k, int ld, int bins, int tile_rows, int kb_floats, bool mn) {
-  if (mn) return MapKey{base, 2 * ld, k, bins, kb_floats / 2, 2 * tile_rows};
-  return MapKey{base, 2 * ld, rows, bins, tile_rows, kb_floats};
+MapKey operand_key(const void* base, int rows, int k, int ld, int bins, int tile_rows, int kb_floats, bool mn,
+                   bool swizzle) {
+  if (mn) return MapKey{base, 2 * ld, k, bins, kb_floats / 2, 2 * tile_rows, false};
+  return MapKey{base, 2 * ld, rows, bins, tile_rows, kb_floats, swizzle};
 }
 struct MapCache {
   static constexpr int kSlots = 32;
@@ -271,7 +293,8 @@ struct MapCache {
         return true;
       }
     CUtensorMap m;
-    if (!make_map(&m, key.base, key.inner_floats, key.rows, key.bins, key.box_rows, key.box_floats)) return false;
+    if (!make_map(&m, key.base, key.inner_floats, key.rows, key.bins, key.box_rows, key.box_floats, key.swizzle))
+      return false;
     const int slot = next;
     next = (next + 1) % kSlots;
     keys[slot] = key;
@@ -288,8 +311,8 @@ cudaError_t launch_wide_as(const ContractParams& p, cudaStream_t stream) {
   using namespace wide;
   using TL = WideTile<WBNC>;
   CUtensorMap map_a, map_b;
-  if (!g_maps.get(operand_key(p.a, p.m, p.k, p.lda, p.bins, WBM, TL::KB, p.a_mn != 0), &map_a) ||
-      !g_maps.get(operand_key(p.b, p.n, p.k, p.ldb, p.bins, WBNC, TL::KB, p.b_mn != 0), &map_b))
+  if (!g_maps.get(operand_key(p.a, p.m, p.k, p.lda, p.bins, WBM, TL::KB, p.a_mn != 0, true), &map_a) ||
+      !g_maps.get(operand_key(p.b, p.n, p.k, p.ldb, p.bins, WBNC, TL::KB, p.b_mn != 0, false), &map_b))
     return cudaErrorInvalidValue;
   WideParams t;
   t.c = p.c;

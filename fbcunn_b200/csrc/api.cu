@@ -1478,34 +1478,55 @@ int fbfftconv_host_sync(fbfftconv_handle* h) {
 
 // ---- sub-steps ---------------------------------------------------------------
 
-int fbfftconv_fft2d(const float* real, void* spectrum, int d1, int d2, int h, int w, int fft_size,
-                    int pad_u, int pad_l, int transposed, fbfftconv_stream stream) {
+namespace {
+
+// `reference`: the spectrum is the reference's frequency tensor (fft_modes_supported sizes, d1 = 1).
+int transform_fft2d(const float* real, float2* spectrum, int d1, int d2, int h, int w, int fft_size, int pad_u,
+                    int pad_l, int transposed, bool reference, fbfftconv_stream stream) {
   if (!real || !spectrum) return fail(FBFFTCONV_ERR_INVALID_ARGUMENT, "null argument");
   if (!valid_fft_size(fft_size)) return fail(FBFFTCONV_ERR_UNSUPPORTED_SIZE, "transform size %d not in {2,4,8,16,32,64,128}", fft_size);
   if (d1 <= 0 || d2 <= 0 || h <= 0 || w <= 0 || pad_u < 0 || pad_l < 0 || h + pad_u > fft_size ||
       w + pad_l > fft_size || d1 > 65535 || d2 > 65535)
     return fail(FBFFTCONV_ERR_INVALID_ARGUMENT, "plane of %dx%d at (%d,%d) does not fit %d", h, w, pad_u, pad_l, fft_size);
-  const FftParams p = forward_params(real, static_cast<float2*>(spectrum), d1, d2, h, w, pad_u, pad_l, transposed, fft_size);
+  FftParams p = forward_params(real, spectrum, d1, d2, h, w, pad_u, pad_l, transposed, fft_size);
+  p.reference = reference;
   FBF_CUDA(launch_forward(&p, 1, fft_size, static_cast<cudaStream_t>(stream)));
   return FBFFTCONV_OK;
 }
 
-int fbfftconv_ifft2d(const void* spectrum, float* real, const float* bias, int d1, int d2, int h,
-                     int w, int fft_size, int off_y, int off_x, int accumulate, int plane_major,
-                     fbfftconv_stream stream) {
+int transform_ifft2d(const float2* spectrum, float* real, const float* bias, int d1, int d2, int h, int w, int fft_size,
+                     int off_y, int off_x, int accumulate, int plane_major, bool reference, fbfftconv_stream stream) {
   if (!real || !spectrum) return fail(FBFFTCONV_ERR_INVALID_ARGUMENT, "null argument");
   if (!valid_fft_size(fft_size)) return fail(FBFFTCONV_ERR_UNSUPPORTED_SIZE, "transform size %d not in {2,4,8,16,32,64,128}", fft_size);
   if (d1 <= 0 || d2 <= 0 || h <= 0 || w <= 0 || off_y < 0 || off_x < 0 || h + off_y > fft_size ||
       w + off_x > fft_size || d1 > 65535 || d2 > 65535)
     return fail(FBFFTCONV_ERR_INVALID_ARGUMENT, "window of %dx%d at (%d,%d) does not fit %d", h, w, off_y, off_x, fft_size);
-  return inverse_transform(inverse_params(static_cast<const float2*>(spectrum), real, bias, d1, d2, h, w, off_y, off_x,
-                                          accumulate != 0, plane_major != 0 ? 2 : 0, fft_size),
-                           nullptr, fft_size, static_cast<cudaStream_t>(stream));
+  FftParams p = inverse_params(spectrum, real, bias, d1, d2, h, w, off_y, off_x, accumulate != 0,
+                               plane_major != 0 ? 2 : 0, fft_size);
+  p.reference = reference;
+  return inverse_transform(p, nullptr, fft_size, static_cast<cudaStream_t>(stream));
+}
+
+}  // namespace
+
+int fbfftconv_fft2d(const float* real, void* spectrum, int d1, int d2, int h, int w, int fft_size,
+                    int pad_u, int pad_l, int transposed, fbfftconv_stream stream) {
+  return transform_fft2d(real, static_cast<float2*>(spectrum), d1, d2, h, w, fft_size, pad_u, pad_l, transposed, false,
+                         stream);
+}
+
+int fbfftconv_ifft2d(const void* spectrum, float* real, const float* bias, int d1, int d2, int h,
+                     int w, int fft_size, int off_y, int off_x, int accumulate, int plane_major,
+                     fbfftconv_stream stream) {
+  return transform_ifft2d(static_cast<const float2*>(spectrum), real, bias, d1, d2, h, w, fft_size, off_y, off_x,
+                          accumulate, plane_major, false, stream);
 }
 
 int fbfftconv_fft2d_reference_layout(const float* real, void* frequency, void* scratch, int planes, int h, int w,
                                      int fft_size, int pad_u, int pad_l, fbfftconv_stream stream) {
   if (!scratch || !frequency) return fail(FBFFTCONV_ERR_INVALID_ARGUMENT, "null argument");
+  if (fft_modes_supported(fft_size))
+    return transform_fft2d(real, static_cast<float2*>(frequency), 1, planes, h, w, fft_size, pad_u, pad_l, 0, true, stream);
   FBF_TRY(fbfftconv_fft2d(real, scratch, 1, planes, h, w, fft_size, pad_u, pad_l, 0, stream));
   FBF_CUDA(launch_spectrum_layout(true, static_cast<const float2*>(scratch), static_cast<float2*>(frequency), planes,
                                   pad4(planes), fft_size, static_cast<cudaStream_t>(stream)));
@@ -1517,6 +1538,9 @@ int fbfftconv_ifft2d_reference_layout(const void* frequency, float* real, void* 
   if (!scratch || !frequency || !real) return fail(FBFFTCONV_ERR_INVALID_ARGUMENT, "null argument");
   if (!valid_fft_size(fft_size)) return fail(FBFFTCONV_ERR_UNSUPPORTED_SIZE, "transform size %d not in {2,4,8,16,32,64,128}", fft_size);
   if (planes <= 0 || planes > 65535) return fail(FBFFTCONV_ERR_INVALID_ARGUMENT, "between 1 and 65535 planes");
+  if (fft_modes_supported(fft_size))
+    return transform_ifft2d(static_cast<const float2*>(frequency), real, nullptr, 1, planes, h, w, fft_size, off_y,
+                            off_x, 0, 0, true, stream);
   FBF_CUDA(launch_spectrum_layout(false, static_cast<const float2*>(frequency), static_cast<float2*>(scratch), planes,
                                   pad4(planes), fft_size, static_cast<cudaStream_t>(stream)));
   return fbfftconv_ifft2d(scratch, real, nullptr, 1, planes, h, w, fft_size, off_y, off_x, 0, 0, stream);

@@ -348,6 +348,7 @@ struct FftParams {
   long long real_row_stride, real_inner_stride;
   int accumulate;         // inverse only: real_out += result
   TileView view;          // thread-per-line sizes of 8 points and more
+  int reference;          // the same sizes, one row: `spec` is the reference's tensor (reference_offset)
 };
 
 // Place of one tile of a view: offset of its image plane, image coordinates of its first element.
@@ -365,6 +366,20 @@ FBF_HD TilePlace tile_place(const TileView& v, int row, int inner) {
   r.x0 = tx * v.sw + v.ox;
   return r;
 }
+// What a kernel's planes and spectrum may be besides planes in memory and the library's half spectrum.
+enum FftMode { kPlanes = 0, kTiles = 1, kReference = 2 };
+
+// The reference's 2-D frequency tensor of 8 to 32 points, (planes, N/2+1, N): rows ky <= N/2 of the full
+// spectrum (test/test_FFTModule.lua:310-342).  Column kx <= N/2 of the half spectrum holds the elements
+// [ky][kx], ky <= N/2, and, conjugated, the elements [N-ky][N-kx] of the other half (0 < kx < N/2).
+// The transforms address it themselves: bound by HBM, a converting kernel doubled the spectrum's traffic and
+// the launches (8192 planes of 32 points there and back: 83 us with it, 42 without).  At 64 and 128 points the
+// tensor is the half spectrum transposed, whose 8-byte pieces a bin-major column step would scatter.
+template <int N>
+FBF_HD long long reference_offset(int plane, int kx) {
+  return (long long)plane * ((N / 2 + 1) * N) + kx;
+}
+
 // log2 of the lanes that copy the rows of a tile w columns wide together.
 FBF_HD int tile_group_shift(int w) { return w <= 8 ? 3 : w <= 16 ? 4 : 5; }
 
@@ -432,11 +447,11 @@ struct Forward {
   }
 
   // Phase 0: real planes -> stage, plane t at stage + t*pitch1 + phase16(plane); warps take planes.
-  // VIEW (here and below): the planes may be tiles of images, staged without a shift.
-  template <bool VIEW = false>
+  // kTiles (here and below): the planes may be tiles of images, staged without a shift.
+  template <int MODE = kPlanes>
   static FBF_HD void load(const FftParams& p, const FftGeom& g, char* smem, int tid, int nthreads,
                           int row, int inner0) {
-    if (VIEW && p.view.nw) return load_tiles(p, g, smem, tid, nthreads, row, inner0);
+    if (MODE == kTiles && p.view.nw) return load_tiles(p, g, smem, tid, nthreads, row, inner0);
     float* stage = reinterpret_cast<float*>(smem + g.off_a);
     const int hw = p.h * p.w;
     // small planes: a warp splits into groups of 8 or 16 lanes that take one plane each
@@ -460,14 +475,14 @@ struct Forward {
   }
 
   // Phase 1a: rows (j, j+hh) of plane t into registers as (re, im), zero outside the plane.
-  template <bool VIEW = false>
+  template <int MODE = kPlanes>
   static FBF_HD void row_fetch(const FftParams& p, const FftGeom& g, const char* smem, int line, int row,
                                int inner0, LineRegs<N>& regs) {
     if (line >= g.lines1) return;
     const float* stage = reinterpret_cast<const float*>(smem + g.off_a);
     const int j = line / T, t = line - j * T;
     const bool live = inner0 + t < p.n_inner;
-    const float* sp = stage + t * g.pitch1 + (VIEW && p.view.nw ? 0 : phase16(plane_ptr(p, row, inner0 + t)));
+    const float* sp = stage + t * g.pitch1 + (MODE == kTiles && p.view.nw ? 0 : phase16(plane_ptr(p, row, inner0 + t)));
     const int ya = j - p.off_y, yb = ya + g.hh;
     const bool va = live && (unsigned)ya < (unsigned)p.h, vb = live && (unsigned)yb < (unsigned)p.h;
     const float* pa = sp + ya * p.w - p.off_x;
@@ -518,6 +533,7 @@ struct Forward {
   }
 
   // Phase 2: transform along y for line2 = kx*T + t and write the spectrum.
+  template <int MODE = kPlanes>
   static FBF_HD void col_pass(const FftParams& p, const FftGeom& g, char* smem, int line, int row,
                               int inner0) {
     if (line >= L::LINES2) return;
@@ -530,6 +546,18 @@ struct Forward {
 #pragma unroll
     for (int y = 0; y < N; ++y) u[y] = y < he ? mid[y * L::PITCH2] : make_float2(0.f, 0.f);
     fft_inreg<N, false>(u);
+    if constexpr (MODE == kReference) {
+      if (inner >= p.n_inner) return;
+      float2* ref = p.spec + reference_offset<N>(inner, kx);
+#pragma unroll
+      for (int ky = 0; ky <= N / 2; ++ky) ref[ky * N] = u[ky];
+      if (kx > 0 && kx < N / 2) {
+        ref += N - 2 * kx;
+#pragma unroll
+        for (int ky = 0; ky <= N / 2; ++ky) ref[ky * N] = make_float2(u[(N - ky) % N].x, -u[(N - ky) % N].y);
+      }
+      return;
+    }
     // 32-bit offsets inside the row: the launcher refuses spectra of 2^31 elements or more
     float2* dst = p.spec + ((long long)kx * p.spec_bin + row * p.spec_row + inner * p.spec_inner);
     const int step = L::KX * (int)p.spec_bin;
@@ -547,6 +575,7 @@ struct Inverse {
   }
 
   // Phase 1: inverse transform along y of line2 = kx*T + t, keep the crop rows.
+  template <int MODE = kPlanes>
   static FBF_HD void col_pass(const FftParams& p, const FftGeom& g, char* smem, int line, int row,
                               int inner0) {
     if (line >= L::LINES2) return;
@@ -556,8 +585,18 @@ struct Inverse {
     const float2* src = p.spec + ((long long)kx * p.spec_bin + row * p.spec_row + inner * p.spec_inner);
     const int step = L::KX * (int)p.spec_bin;
     float2 u[N];
+    if constexpr (MODE == kReference) {
+      const float2* ref = p.spec + reference_offset<N>(inner, kx);
+      const float2* mirror = p.spec + reference_offset<N>(inner, (N - kx) % N);
 #pragma unroll
-    for (int ky = 0; ky < N; ++ky) u[ky] = live ? src[ky * step] : make_float2(0.f, 0.f);
+      for (int ky = 0; ky < N; ++ky) {
+        const float2 v = !live ? make_float2(0.f, 0.f) : ky <= N / 2 ? ref[ky * N] : mirror[(N - ky) * N];
+        u[ky] = ky <= N / 2 ? v : make_float2(v.x, -v.y);
+      }
+    } else {
+#pragma unroll
+      for (int ky = 0; ky < N; ++ky) u[ky] = live ? src[ky * step] : make_float2(0.f, 0.f);
+    }
     fft_inreg<N, true>(u);
     // row y of the square lands in row y - off_y of mid
     float2* mid = reinterpret_cast<float2*>(smem + g.off_b) + line - p.off_y * L::PITCH2;
@@ -586,14 +625,14 @@ struct Inverse {
 
   // Phase 2b: inverse transform along x, stage the crop columns as real rows, plane t at
   // stage + t*pitch1 + phase16(its destination).
-  template <bool VIEW = false>
+  template <int MODE = kPlanes>
   static FBF_HD void row_pass(const FftParams& p, const FftGeom& g, char* smem, int line, int row,
                               int inner0, LineRegs<N>& regs) {
     if (line >= g.lines1) return;
     float* stage = reinterpret_cast<float*>(smem + g.off_a);
     const int j = line / T, t = line - j * T;
     const bool has_b = (j + g.hh) < g.he;
-    const int shift = VIEW && p.view.nw ? 0 : phase16(plane_ptr(p, g, row, inner0 + t));
+    const int shift = MODE == kTiles && p.view.nw ? 0 : phase16(plane_ptr(p, g, row, inner0 + t));
     float* sa = stage + t * g.pitch1 + shift + j * g.we - p.off_x;
     float* sb = sa + g.hh * g.we;
     const unsigned we = (unsigned)g.we;
@@ -653,10 +692,10 @@ struct Inverse {
   }
 
   // Phase 3: staged planes -> global in 16-byte pieces, bias added per plane; warps take planes.
-  template <bool VIEW = false>
+  template <int MODE = kPlanes>
   static FBF_HD void store(const FftParams& p, const FftGeom& g, const char* smem, int tid,
                            int nthreads, int row, int inner0) {
-    if (VIEW && p.view.nw) return store_tiles(p, g, smem, tid, nthreads, row, inner0);
+    if (MODE == kTiles && p.view.nw) return store_tiles(p, g, smem, tid, nthreads, row, inner0);
     const float* stage = reinterpret_cast<const float*>(smem + g.off_a);
     const int per_plane = g.he * g.we;
     const int lp_shift = copy_group_shift(per_plane);

@@ -110,8 +110,9 @@ __device__ __forceinline__ void with_operand(const FftBatch<OPS>& b, int tile, B
   }
 }
 
-// VIEW: planes of some operand are tiles of images (a kernel of its own, so that the others stay as they are).
-template <int N, int T, int OPS, bool VIEW>
+// MODE: planes of some operand are tiles of images, or the spectrum is the reference's tensor (kernels of their
+// own, so that the others stay as they are).
+template <int N, int T, int OPS, int MODE>
 __global__ void __launch_bounds__(block_threads<N, T>())
 fft2d_forward_kernel(const __grid_constant__ FftBatch<OPS> b) {
   extern __shared__ __align__(16) char smem[];
@@ -120,18 +121,18 @@ fft2d_forward_kernel(const __grid_constant__ FftBatch<OPS> b) {
   with_operand(b, blockIdx.x, [&](const FftParams& p, const FftGeom& g, int tile, int tiles_x) {
     const int row = tile / tiles_x;
     const int inner0 = (tile - row * tiles_x) * T;
-    Forward<N, T>::template load<VIEW>(p, g, smem, tid, blockDim.x, row, inner0);
+    Forward<N, T>::template load<MODE>(p, g, smem, tid, blockDim.x, row, inner0);
     __syncthreads();
     LineRegs<N> regs;
-    Forward<N, T>::template row_fetch<VIEW>(p, g, smem, tid, row, inner0, regs);
+    Forward<N, T>::template row_fetch<MODE>(p, g, smem, tid, row, inner0, regs);
     __syncthreads();  // the column buffer aliases the staged planes
     Forward<N, T>::row_pass(g, smem, tid, regs);
     __syncthreads();
-    Forward<N, T>::col_pass(p, g, smem, tid, row, inner0);
+    Forward<N, T>::template col_pass<MODE>(p, g, smem, tid, row, inner0);
   });
 }
 
-template <int N, int T, int OPS, bool VIEW>
+template <int N, int T, int OPS, int MODE>
 __global__ void __launch_bounds__(block_threads<N, T>())
 fft2d_inverse_kernel(const __grid_constant__ FftBatch<OPS> b) {
   extern __shared__ __align__(16) char smem[];
@@ -144,14 +145,14 @@ fft2d_inverse_kernel(const __grid_constant__ FftBatch<OPS> b) {
   with_operand(b, (int)blockIdx.x - b.sum_blocks, [&](const FftParams& p, const FftGeom& g, int tile, int tiles_x) {
     const int row = tile / tiles_x;
     const int inner0 = (tile - row * tiles_x) * T;
-    Inverse<N, T>::col_pass(p, g, smem, tid, row, inner0);
+    Inverse<N, T>::template col_pass<MODE>(p, g, smem, tid, row, inner0);
     __syncthreads();
     LineRegs<N> regs;
     Inverse<N, T>::row_fetch(g, smem, tid, regs);
     __syncthreads();  // the staged output aliases the column buffer
-    Inverse<N, T>::template row_pass<VIEW>(p, g, smem, tid, row, inner0, regs);
+    Inverse<N, T>::template row_pass<MODE>(p, g, smem, tid, row, inner0, regs);
     __syncthreads();
-    Inverse<N, T>::template store<VIEW>(p, g, smem, tid, blockDim.x, row, inner0);
+    Inverse<N, T>::template store<MODE>(p, g, smem, tid, blockDim.x, row, inner0);
   });
 }
 
@@ -352,11 +353,12 @@ cudaError_t run_batch(bool inverse, const FftParams* ops, int count, const RowSu
   FftBatch<OPS> b{};
   long long tiles = 0;
   int smem = 0;
-  bool view = false;
+  int mode = kPlanes;
   for (int i = 0; i < OPS; ++i) {
     if (i < count) {
       b.p[i] = ops[i];
-      view |= ops[i].view.nw != 0;
+      if (ops[i].view.nw) mode = kTiles;
+      if (ops[i].reference) mode = kReference;
       b.g[i] = inverse ? inverse_geom(N, T, ops[i].h, ops[i].w)
                        : forward_geom(N, T, ops[i].h, ops[i].w, ops[i].off_y, ops[i].off_x);
       b.tiles_x[i] = ((inverse ? ops[i].n_inner : ops[i].kc) + T - 1) / T;
@@ -379,11 +381,16 @@ cudaError_t run_batch(bool inverse, const FftParams* ops, int count, const RowSu
     blocks = persistent_blocks(N, tiles);
   } else {
     if (threads != block_threads<N, T>()) return cudaErrorInvalidConfiguration;
-    kernel = inverse ? fft2d_inverse_kernel<N, T, OPS, false> : fft2d_forward_kernel<N, T, OPS, false>;
+    kernel = inverse ? fft2d_inverse_kernel<N, T, OPS, kPlanes> : fft2d_forward_kernel<N, T, OPS, kPlanes>;
     if constexpr (N >= 8)
-      if (view) kernel = inverse ? fft2d_inverse_kernel<N, T, OPS, true> : fft2d_forward_kernel<N, T, OPS, true>;
+      if (mode == kTiles)
+        kernel = inverse ? fft2d_inverse_kernel<N, T, OPS, kTiles> : fft2d_forward_kernel<N, T, OPS, kTiles>;
+    if constexpr (N >= 8 && OPS == 1)
+      if (mode == kReference)
+        kernel = inverse ? fft2d_inverse_kernel<N, T, 1, kReference> : fft2d_forward_kernel<N, T, 1, kReference>;
   }
-  if (view && !tile_view_supported(N)) return cudaErrorInvalidConfiguration;
+  if (mode != kPlanes && !fft_modes_supported(N)) return cudaErrorInvalidConfiguration;
+  if (mode == kReference && (OPS > 1 || ops[0].n_rows != 1 || ops[0].view.nw)) return cudaErrorInvalidConfiguration;
   cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
   if (e != cudaSuccess) return e;
   e = launch_dependent(kernel, dim3((unsigned)(blocks + b.sum_blocks)), threads, smem, stream, b);
@@ -498,13 +505,13 @@ cudaError_t launch_fft1d(bool inverse, const float* real_in, float* real_out, fl
 namespace {
 
 // The reference's 2-D frequency tensor (planes, N/2+1, N, 2) holds, for 8 <= N <= 32, rows ky <= N/2
-// of the full spectrum (element [ky][kx] = X[ky][kx] for every kx), and for the other sizes the half
-// spectrum along x stored transposed (element [kx][ky] = X[ky][kx], kx <= N/2)
-// (test/test_FFTModule.lua:310-342).  The library's half spectrum is [bin = ky*(N/2+1) + kx][plane],
-// kx <= N/2; the missing half follows from X[ky][kx] = conj(X[-ky][-kx]).
+// of the full spectrum, which the transforms store and load themselves (kReference), and for the other
+// sizes the half spectrum along x stored transposed (element [kx][ky] = X[ky][kx], kx <= N/2)
+// (test/test_FFTModule.lua:310-342), which the kernels below convert from and to the library's half
+// spectrum [bin = ky*(N/2+1) + kx][plane].
 __global__ void __launch_bounds__(256)
 spectrum_to_reference_kernel(const float2* __restrict__ spec, float2* __restrict__ ref, long long planes, int kc,
-                             int N, int transposed) {
+                             int N) {
   grid_dependency_wait();
   const int KX = N / 2 + 1;
   const long long per_plane = (long long)KX * N;
@@ -512,30 +519,14 @@ spectrum_to_reference_kernel(const float2* __restrict__ spec, float2* __restrict
        i += (long long)gridDim.x * blockDim.x) {
     const long long p = i / per_plane;
     const int r = (int)(i - p * per_plane);
-    const int a = r / N, b = r - a * N;  // element [a][b] of the reference tensor, a <= N/2
-    int ky, kx;
-    bool conj = false;
-    if (transposed) {
-      kx = a;
-      ky = b;
-    } else {
-      ky = a;
-      kx = b;
-      if (kx > N / 2) {
-        ky = (N - ky) % N;
-        kx = N - kx;
-        conj = true;
-      }
-    }
-    float2 v = spec[((long long)ky * KX + kx) * kc + p];
-    if (conj) v.y = -v.y;
-    ref[i] = v;
+    const int a = r / N, b = r - a * N;  // element [kx = a][ky = b]
+    ref[i] = spec[((long long)b * KX + a) * kc + p];
   }
 }
 
 __global__ void __launch_bounds__(256)
 reference_to_spectrum_kernel(const float2* __restrict__ ref, float2* __restrict__ spec, long long planes, int kc,
-                             int N, int transposed) {
+                             int N) {
   grid_dependency_wait();
   const int KX = N / 2 + 1;
   const long long bins = (long long)KX * N;
@@ -546,15 +537,7 @@ reference_to_spectrum_kernel(const float2* __restrict__ ref, float2* __restrict_
     float2 v = make_float2(0.f, 0.f);  // the padding planes of the library's layout are zero
     if (p < planes) {
       const int ky = (int)(bin / KX), kx = (int)(bin - (long long)ky * KX);
-      const float2* plane = ref + p * bins;
-      if (transposed) {
-        v = plane[kx * N + ky];
-      } else if (ky <= N / 2) {
-        v = plane[ky * N + kx];
-      } else {  // X[ky][kx] = conj(X[N-ky][(N-kx) % N])
-        v = plane[(N - ky) * N + (N - kx) % N];
-        v.y = -v.y;
-      }
+      v = ref[p * bins + kx * N + ky];
     }
     spec[i] = v;
   }
@@ -564,12 +547,11 @@ reference_to_spectrum_kernel(const float2* __restrict__ ref, float2* __restrict_
 
 cudaError_t launch_spectrum_layout(bool to_reference, const float2* src, float2* dst, long long planes, int kc, int N,
                                    cudaStream_t stream) {
-  const bool transposed = N < 8 || N > 32;
   const long long total = to_reference ? planes * (N / 2 + 1) * N : (long long)(N / 2 + 1) * N * kc;
   const long long want = (total + 255) / 256, cap = (long long)sm_count() * 16;
   const int blocks = (int)(want < 1 ? 1 : want < cap ? want : cap);
   const cudaError_t e = launch_dependent(to_reference ? spectrum_to_reference_kernel : reference_to_spectrum_kernel,
-                                         dim3(blocks), 256, 0, stream, src, dst, planes, kc, N, (int)transposed);
+                                         dim3(blocks), 256, 0, stream, src, dst, planes, kc, N);
   count_launch();
   return e;
 }

@@ -63,8 +63,9 @@ struct RowSum {
 };
 
 constexpr int kMaxFftOps = 3;
-// Transform sizes whose kernels take tiles of images as planes (FftParams::view).
-constexpr bool tile_view_supported(int N) { return N >= 8 && N <= 32; }
+// Transform sizes whose kernels take tiles of images as planes (FftParams::view) and the reference's frequency
+// tensor as spectrum (FftParams::reference).
+constexpr bool fft_modes_supported(int N) { return N >= 8 && N <= 32; }
 // Transforms of up to kMaxFftOps operands in one launch (all of the same size N).
 cudaError_t launch_forward(const FftParams* ops, int count, int N, cudaStream_t stream);
 cudaError_t launch_inverse(const FftParams* ops, int count, const RowSum* sum, int N, cudaStream_t stream);
@@ -74,8 +75,9 @@ cudaError_t launch_fft1d(bool inverse, const float* real_in, float* real_out, fl
 // The 1-D transforms of 64, 128 and 256 points (fft1d_lines.cu), same arguments.
 cudaError_t launch_fft1d_lines(bool inverse, const float* real_in, float* real_out, float2* spec, long long rows,
                                int n, int N, int offset, cudaStream_t stream);
-// Between the library's half spectrum [bin][plane (padded to kc)] and the reference's 2-D frequency
-// tensor (planes, N/2+1, N, 2) (nn.FFTWrapper, test/test_FFTModule.lua:310-342).
+// Between the library's half spectrum [bin][plane (padded to kc)] and the reference's 2-D frequency tensor
+// (planes, N/2+1, N, 2) of the sizes that store it transposed (nn.FFTWrapper, test/test_FFTModule.lua:310-342):
+// all that fft_modes_supported does not name.
 cudaError_t launch_spectrum_layout(bool to_reference, const float2* src, float2* dst, long long planes, int kc, int N,
                                    cudaStream_t stream);
 

@@ -254,7 +254,7 @@ int fbfftconv_tiled_create(const fbfftconv_desc* desc, int tile_h, int tile_w, f
     delete t;
     return rc;
   }
-  t->views = tile_view_supported(fbfftconv_fft_size(t->inner));
+  t->views = fft_modes_supported(fbfftconv_fft_size(t->inner));
   t->save_grad_input = !(d.flags & FBFFTCONV_REUSE_OUTPUT) && ceil_div(d.input_h, t->sh) <= t->nh &&
                        ceil_div(d.input_w, t->sw) <= t->nw;
   t->device = d.device;

@@ -60,14 +60,21 @@ void run_forward(const FftParams& p) {
             CoopForward<N, T>::template col_step2<false>(p, g, smem.data(), tid, nth, row, inner0);
       } else {
         for (int tid = 0; tid < g.threads; ++tid)
-          Forward<N, T>::template load<true>(p, g, smem.data(), tid, g.threads, row, inner0);
+          Forward<N, T>::template load<kTiles>(p, g, smem.data(), tid, g.threads, row, inner0);
         for (int tid = 0; tid < g.threads; ++tid)
-          Forward<N, T>::template row_fetch<true>(p, g, smem.data(), tid, row, inner0, regs[tid]);
+          Forward<N, T>::template row_fetch<kTiles>(p, g, smem.data(), tid, row, inner0, regs[tid]);
         std::memset(smem.data(), 0xFF, smem.size());  // aliasing: the row buffer is dead now
         for (int tid = 0; tid < g.threads; ++tid)
           Forward<N, T>::row_pass(g, smem.data(), tid, regs[tid]);
         for (int tid = 0; tid < g.threads; ++tid)
-          Forward<N, T>::col_pass(p, g, smem.data(), tid, row, inner0);
+          if constexpr (N >= 8) {
+            if (p.reference)
+              Forward<N, T>::template col_pass<kReference>(p, g, smem.data(), tid, row, inner0);
+            else
+              Forward<N, T>::col_pass(p, g, smem.data(), tid, row, inner0);
+          } else {
+            Forward<N, T>::col_pass(p, g, smem.data(), tid, row, inner0);
+          }
       }
     }
   }
@@ -109,14 +116,21 @@ void run_inverse(const FftParams& p, int oh, int ow) {
         }
       } else {
         for (int tid = 0; tid < g.threads; ++tid)
-          Inverse<N, T>::col_pass(p, g, smem.data(), tid, row, inner0);
+          if constexpr (N >= 8) {
+            if (p.reference)
+              Inverse<N, T>::template col_pass<kReference>(p, g, smem.data(), tid, row, inner0);
+            else
+              Inverse<N, T>::col_pass(p, g, smem.data(), tid, row, inner0);
+          } else {
+            Inverse<N, T>::col_pass(p, g, smem.data(), tid, row, inner0);
+          }
         for (int tid = 0; tid < g.threads; ++tid)
           Inverse<N, T>::row_fetch(g, smem.data(), tid, regs[tid]);
         std::memset(smem.data() + g.off_b, 0xFF, smem.size() - g.off_b);  // mid is dead now
         for (int tid = 0; tid < g.threads; ++tid)
-          Inverse<N, T>::template row_pass<true>(p, g, smem.data(), tid, row, inner0, regs[tid]);
+          Inverse<N, T>::template row_pass<kTiles>(p, g, smem.data(), tid, row, inner0, regs[tid]);
         for (int tid = 0; tid < g.threads; ++tid)
-          Inverse<N, T>::template store<true>(p, g, smem.data(), tid, g.threads, row, inner0);
+          Inverse<N, T>::template store<kTiles>(p, g, smem.data(), tid, g.threads, row, inner0);
       }
     }
   }
@@ -273,6 +287,21 @@ int hostcheck_fft_tiles(int inverse, float* images, float* spec, const float* bi
   p.kc = kc;
   set_layout(p, N, 0);
   return dispatch(inverse != 0, p, N, T, p.h, p.w);
+}
+
+// The spectrum is the reference's frequency tensor (planes, N/2+1, N).
+int hostcheck_fft_reference(int inverse, float* real, float* spec, int N, int T, int h, int w, int off_y, int off_x,
+                            int planes) {
+  FftParams p{};
+  p.real_in = real;
+  p.real_out = real;
+  p.spec = reinterpret_cast<float2*>(spec);
+  p.h = h; p.w = w; p.off_y = off_y; p.off_x = off_x;
+  p.n_rows = 1; p.n_inner = planes; p.kc = (planes + 3) / 4 * 4;
+  p.real_inner_stride = 1;
+  p.reference = 1;
+  set_layout(p, N, 0);
+  return dispatch(inverse != 0, p, N, T, h, w);
 }
 
 int hostcheck_forward_smem_bytes(int N, int T, int h, int w, int pad_u, int pad_l) {

@@ -202,3 +202,27 @@ def test_tiles_of_images(hc, tile, H, W, pU, pL, kH, kW, by_inner):
     h, w = min(H, nh * sh), min(W, nw * sw)
     assert np.array_equal(out[:, :, :h, :w], whole[:, :, :h, :w])
     assert np.isnan(out[:, :, h:]).all() and np.isnan(out[:, :, :, w:]).all()
+
+
+@pytest.mark.parametrize("planes", (1, 5, 17))
+@pytest.mark.parametrize("N", (8, 16, 32))
+def test_reference_tensor(hc, N, planes):
+    """The transforms that store and load the reference's frequency tensor (planes, N/2+1, N) themselves."""
+    T = 16 if N <= 16 else 8
+    rng = np.random.default_rng(N + planes)
+    for h, w, oy, ox in [(N, N, 0, 0), (N - 3, N - 2, 1, 2)]:
+        x = rng.standard_normal((planes, h, w)).astype(np.float32)
+        spec = np.full((planes, N // 2 + 1, N, 2), np.nan, np.float32)
+        back = np.full_like(x, np.nan)
+
+        def run(inverse, real):
+            assert hc.hostcheck_fft_reference(inverse, real.ctypes.data_as(ctypes.c_void_p),
+                                              spec.ctypes.data_as(ctypes.c_void_p), N, T, h, w, oy, ox, planes) == 0
+
+        run(0, x)
+        square = np.zeros((planes, N, N))
+        square[:, oy:oy + h, ox:ox + w] = x
+        ref = np.fft.fft2(square)[:, :N // 2 + 1]
+        assert np.abs(spec[..., 0] + 1j * spec[..., 1] - ref).max() <= 5e-6 * np.abs(ref).max()
+        run(1, back)
+        assert np.abs(back - N * N * x).max() <= 5e-6 * N * N * np.abs(x).max()

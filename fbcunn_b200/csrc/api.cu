@@ -1522,11 +1522,31 @@ int fbfftconv_ifft2d(const void* spectrum, float* real, const float* bias, int d
                           accumulate, plane_major, false, stream);
 }
 
+namespace {
+
+size_t reference_bytes(int planes, int N) { return (size_t)planes * (N / 2 + 1) * N * sizeof(float2); }
+// Whether the real planes and the reference's frequency tensor share memory.  The transforms that address that
+// tensor themselves read and write in no order across blocks, so such a call goes through the scratch block.
+bool shares_memory(const float* real, const void* frequency, int planes, int h, int w, int N) {
+  if (planes <= 0 || h <= 0 || w <= 0) return false;  // refused by the transform
+  const uintptr_t r = reinterpret_cast<uintptr_t>(real), f = reinterpret_cast<uintptr_t>(frequency);
+  return r < f + reference_bytes(planes, N) && f < r + (size_t)planes * h * w * sizeof(float);
+}
+
+}  // namespace
+
 int fbfftconv_fft2d_reference_layout(const float* real, void* frequency, void* scratch, int planes, int h, int w,
                                      int fft_size, int pad_u, int pad_l, fbfftconv_stream stream) {
   if (!scratch || !frequency) return fail(FBFFTCONV_ERR_INVALID_ARGUMENT, "null argument");
-  if (fft_modes_supported(fft_size))
-    return transform_fft2d(real, static_cast<float2*>(frequency), 1, planes, h, w, fft_size, pad_u, pad_l, 0, true, stream);
+  if (fft_modes_supported(fft_size)) {
+    const bool in_place = shares_memory(real, frequency, planes, h, w, fft_size);
+    FBF_TRY(transform_fft2d(real, static_cast<float2*>(in_place ? scratch : frequency), 1, planes, h, w, fft_size,
+                            pad_u, pad_l, 0, true, stream));
+    if (in_place)
+      FBF_CUDA(cudaMemcpyAsync(frequency, scratch, reference_bytes(planes, fft_size), cudaMemcpyDeviceToDevice,
+                               static_cast<cudaStream_t>(stream)));
+    return FBFFTCONV_OK;
+  }
   FBF_TRY(fbfftconv_fft2d(real, scratch, 1, planes, h, w, fft_size, pad_u, pad_l, 0, stream));
   FBF_CUDA(launch_spectrum_layout(true, static_cast<const float2*>(scratch), static_cast<float2*>(frequency), planes,
                                   pad4(planes), fft_size, static_cast<cudaStream_t>(stream)));
@@ -1538,9 +1558,15 @@ int fbfftconv_ifft2d_reference_layout(const void* frequency, float* real, void* 
   if (!scratch || !frequency || !real) return fail(FBFFTCONV_ERR_INVALID_ARGUMENT, "null argument");
   if (!valid_fft_size(fft_size)) return fail(FBFFTCONV_ERR_UNSUPPORTED_SIZE, "transform size %d not in {2,4,8,16,32,64,128}", fft_size);
   if (planes <= 0 || planes > 65535) return fail(FBFFTCONV_ERR_INVALID_ARGUMENT, "between 1 and 65535 planes");
-  if (fft_modes_supported(fft_size))
+  if (fft_modes_supported(fft_size)) {
+    if (shares_memory(real, frequency, planes, h, w, fft_size)) {
+      FBF_CUDA(cudaMemcpyAsync(scratch, frequency, reference_bytes(planes, fft_size), cudaMemcpyDeviceToDevice,
+                               static_cast<cudaStream_t>(stream)));
+      frequency = scratch;
+    }
     return transform_ifft2d(static_cast<const float2*>(frequency), real, nullptr, 1, planes, h, w, fft_size, off_y,
                             off_x, 0, 0, true, stream);
+  }
   FBF_CUDA(launch_spectrum_layout(false, static_cast<const float2*>(frequency), static_cast<float2*>(scratch), planes,
                                   pad4(planes), fft_size, static_cast<cudaStream_t>(stream)));
   return fbfftconv_ifft2d(scratch, real, nullptr, 1, planes, h, w, fft_size, off_y, off_x, 0, 0, stream);

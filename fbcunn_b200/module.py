@@ -40,6 +40,12 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
     return t.data_ptr() if t is not None else None
 
 
+def _share_memory(a: torch.Tensor, b: torch.Tensor) -> bool:
+    """Whether two contiguous tensors overlap."""
+    return (a.data_ptr() < b.data_ptr() + b.numel() * b.element_size()
+            and b.data_ptr() < a.data_ptr() + a.numel() * a.element_size())
+
+
 def _device_index(device: torch.device) -> int:
     return device.index if device.index is not None else torch.cuda.current_device()
 
@@ -428,14 +434,19 @@ class FFTWrapper:
         assert frequency.shape[-3] == n_fft // 2 + 1
         h, w = time.shape[-2:]
         planes = time.numel() // (h * w)
-        scratch = self._scratch(planes, n_fft, time.device)
+        scratch = self._scratch(planes, n_fft, time, frequency)
         capi.check(capi.lib().fbfftconv_fft2d_reference_layout(
             _ptr(time), _ptr(frequency), _ptr(scratch), planes, h, w, n_fft, self.padUp, self.padLeft, stream))
         return frequency
 
-    def _scratch(self, planes, n_fft, device):
-        """The library's own half spectrum of `planes` planes (a kernel converts it to / from the
-        reference's tensor); kept between calls of the same size."""
+    def _scratch(self, planes, n_fft, time, frequency):
+        """The block that the library goes through where it does not transform between the two tensors
+        directly: its own half spectrum of `planes` planes, which a kernel converts to / from the reference's
+        tensor, and for transforms in place.  Kept between calls of the same size.  Elsewhere the block is not
+        touched: `frequency` stands in for it."""
+        if self._half_along_rows(n_fft) and not _share_memory(time, frequency):
+            return frequency
+        device = time.device
         need = (n_fft // 2 + 1) * n_fft * ((planes + 3) // 4 * 4) * 8  # fbfftconv_spectrum_bytes(n_fft, 1, planes)
         buf = getattr(self, "_scratch_buf", None)
         if buf is None or buf.numel() < need or buf.device != device:
@@ -457,7 +468,7 @@ class FFTWrapper:
         n_fft = frequency.shape[-2]
         h, w = time.shape[-2:]
         planes = time.numel() // (h * w)
-        scratch = self._scratch(planes, n_fft, time.device)
+        scratch = self._scratch(planes, n_fft, time, frequency)
         capi.check(capi.lib().fbfftconv_ifft2d_reference_layout(
             _ptr(frequency), _ptr(time), _ptr(scratch), planes, h, w, n_fft, self.padUp, self.padLeft, stream))
         return time

@@ -236,7 +236,8 @@ int fbfftconv_ifft2d(const void* spectrum, float* real, const float* bias, int d
  * [ky][kx] = X[ky][kx], ky <= N/2, every kx; for the other sizes the half spectrum along x stored
  * transposed, element [kx][ky] = X[ky][kx], kx <= N/2 (test/test_FFTModule.lua:310-342).  `planes`
  * real planes of h x w (at most 65535); `scratch` holds fbfftconv_spectrum_bytes(fft_size, 1, planes)
- * bytes for the library's own layout, which a kernel converts at 64 and 128 (and 2 and 4) points; never null. */
+ * bytes, never null: the library's own layout, which a kernel converts, at 64 and 128 (and 2 and 4) points, and a
+ * copy of the frequency tensor where it shares memory with `real` (a transform in place); else it is not touched. */
 int fbfftconv_fft2d_reference_layout(const float* real, void* frequency, void* scratch, int planes, int h, int w,
                                      int fft_size, int pad_u, int pad_l, fbfftconv_stream stream);
 int fbfftconv_ifft2d_reference_layout(const void* frequency, float* real, void* scratch, int planes, int h, int w,

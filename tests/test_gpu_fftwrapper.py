@@ -69,3 +69,24 @@ def test_2d_reference_layout(n, batch):
     back = torch.full_like(time, float("nan"))
     w.ffti_reference_layout(back, freq, len(batch))
     assert np.abs(back.cpu().numpy() / (n * n) - x).max() <= TOL * n * np.abs(x).max()
+
+
+@pytest.mark.parametrize("planes", [1, 9, 700])
+@pytest.mark.parametrize("n", [4, 8, 16, 32, 64])
+def test_2d_in_place(n, planes):
+    """The real planes in the frequency tensor's own memory, at its start and at its end: the transform reads
+    its input as it was before the call."""
+    w = FFTWrapper("fbfft", 0, 0)
+    x = torch.randn(planes, n, n, device="cuda", generator=torch.Generator(device="cuda").manual_seed(n + planes))
+    freq = torch.empty(planes, n // 2 + 1, n, 2, device="cuda")
+    w.fft_reference_layout(x, freq, 1)
+    back = torch.empty_like(x)
+    w.ffti_reference_layout(back, freq, 1)
+    for first in (0, freq.numel() - x.numel()):
+        shared = torch.full_like(freq, float("nan"))
+        time = shared.view(-1)[first:first + x.numel()].view_as(x)
+        time.copy_(x)
+        w.fft_reference_layout(time, shared, 1)
+        assert torch.equal(shared, freq)
+        w.ffti_reference_layout(time, shared, 1)
+        assert torch.equal(time, back)

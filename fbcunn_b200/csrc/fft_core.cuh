@@ -238,15 +238,34 @@ static inline bool cooperative(int N) { return N > 32; }
 // 5-10 % faster than 16); 8- and 16-point ones are fastest at 16; the cooperative sizes take what lets two
 // blocks share an SM's memory.
 constexpr int fft_tile(int N) { return N > 64 ? 1 : N > 32 ? 4 : N > 16 ? 8 : 16; }
-// Threads of a cooperative block and blocks per SM.  With the column buffer alone in shared memory (69 / 74 KB)
-// three blocks fit an SM, but what bounds these kernels is instruction issue and the latency of a thread's own
-// chain: below 128 registers (three blocks of 192 or 256 threads) spills through the little L1 that is left cost
-// more than the extra warps bring.  Step of a first layer (128 x 3 -> 96 planes of 128 x 128) and of a 64-pixel
-// layer (128 x 64 -> 128 planes), us: 160 x 3 1572 / 1396, 192 x 2 1584 / 1269, 256 x 2 1594 / 1256, 128 x 3
-// 1597 / 1399, 192 x 3 1771 / 1356, 256 x 3 2063 / 1340 (two blocks of 256 threads with a row buffer and block
-// barriers between the row steps: 1626 / 1320; this choice per size: 1556 / 1261).
-constexpr int coop_threads(int N) { return N > 64 ? 160 : 256; }
-constexpr int coop_blocks(int N) { return N > 64 ? 3 : 2; }
+// Threads of a cooperative block, blocks per SM, and whether the blocks are persistent or one per tile.  With the
+// column buffer alone in shared memory (69 KB at 128 points, 74 at 64) two or three blocks fit an SM; what bounds
+// the plane-major kernels is instruction issue and the latency of a thread's own chain, and a shape below 128
+// registers a thread spills.  Bin-major spectra are bound by their 8- and 32-byte pieces: the blocks that share a
+// sector (neighbouring tiles) have to meet it while it is in L2.  Persistent blocks drift apart without bound,
+// blocks handed out in the order of their tiles do not.  (The 128-point inverse, whose loads wait on nothing
+// else, runs a little better persistent.)
+// Stand-alone transforms, us, 160 x 3 / 192 x 2 / 224 x 2 / 256 x 2 persistent, then 160 x 3 / 192 x 2 / 224 x 2 /
+// 256 x 2 with a block per tile:
+//   128 points, plane-major, 12288 planes of 118 x 118: forward 441 / 492 / 486 / 460, inverse 485 / 492 / 526 / 477;
+//     of 70 x 66: forward 330 / 377 / 401 / 396, inverse 358 / 389 / 422 / 409
+//   128 points, bin-major, 128 x 32 planes of 118 x 118: forward 561 / 490 / 512 / 483, 366 / 377 / 371 / 363;
+//     inverse 440 / 295 / 307 / 295, 444 / 301 / 307 / 303; 256 x 64 planes of 11 x 11: forward 2785 / 2467 / 2378 /
+//     2507, 1350 / 1116 / 1083 / 1112; inverse 1895 / 823 / 850 / 855, 1428 / 829 / 855 / 852
+//   64 points, plane-major, 12288 planes of 56 x 56: forward 135 / 152 / 141 / 140, inverse 141 / 135 / 131 / 132;
+//     of 64 x 64: forward 156 / 164 / 168 / 148, inverse 160 / 145 / 150 / 139
+//   64 points, bin-major, 256 x 64 planes of 64 x 64: forward 227 / 235 / 242 / 211, 219 / 234 / 238 / 205;
+//     inverse 262 / 225 / 234 / 219, 258 / 223 / 223 / 211; of 9 x 9: forward 158 / 150 / 145 / 131, 129 / 134 / 129 /
+//     125; inverse 186 / 171 / 170 / 164, 178 / 150 / 154 / 152
+struct CoopShape {
+  int threads, blocks;
+  bool persistent;
+};
+constexpr CoopShape coop_shape(int N, bool inverse, bool plane_major) {
+  if (N <= 64) return CoopShape{256, 2, plane_major};
+  if (plane_major) return CoopShape{160, 3, true};
+  return inverse ? CoopShape{192, 2, true} : CoopShape{256, 2, false};
+}
 
 // Thread-per-line kernels (N <= 32): region A = the T real planes as they lie in global
 // memory (pitch1 floats apart), region B = column buffer [y][kx*T + t]; they alias (a thread
@@ -275,7 +294,7 @@ constexpr int coop_mid_pitch(int cols) { return (cols + 11) / 16 * 16 + 4; }
 constexpr int coop_plane_stride(int kx, int T) { return T == 1 ? kx : (kx + 11) / 16 * 16 + 4; }
 
 // `plane_elems`: elements of one real plane as it lies in global memory.
-static inline FftGeom make_geom(int N, int T, int he, int we, int plane_elems, bool inverse) {
+static inline FftGeom make_geom(int N, int T, int he, int we, int plane_elems, bool inverse, bool plane_major) {
   FftGeom g;
   g.N = N;
   g.T = T;
@@ -299,16 +318,16 @@ static inline FftGeom make_geom(int N, int T, int he, int we, int plane_elems, b
     g.pitch2 = coop_mid_pitch(T * coop_plane_stride(N / 2 + 1, T));  // = CoopLayout::PITCH2
     g.off_b = 0;
     g.smem_bytes = N * g.pitch2 * 8;
-    g.threads = coop_threads(N);
+    g.threads = coop_shape(N, inverse, plane_major).threads;
   }
   return g;
 }
 
-static inline FftGeom forward_geom(int N, int T, int h, int w, int pad_u, int pad_l) {
-  return make_geom(N, T, h + pad_u, w + pad_l, h * w, false);
+static inline FftGeom forward_geom(int N, int T, int h, int w, int pad_u, int pad_l, bool plane_major = false) {
+  return make_geom(N, T, h + pad_u, w + pad_l, h * w, false, plane_major);
 }
-static inline FftGeom inverse_geom(int N, int T, int oh, int ow) {
-  return make_geom(N, T, oh, ow, oh * ow, true);
+static inline FftGeom inverse_geom(int N, int T, int oh, int ow, bool plane_major = false) {
+  return make_geom(N, T, oh, ow, oh * ow, true, plane_major);
 }
 
 // ---------------------------------------------------------------------------
@@ -745,7 +764,6 @@ struct CoopLayout {
   }
   static constexpr int PITCH2 = coop_mid_pitch(T * KXP);  // mid row pitch (float2)
   static_assert(N1 == 8, "the residue pairing below is written for eight residues");
-  static_assert(coop_threads(N) % 32 == 0, "whole warps");
   // Between its two steps a row line lies where its result goes: values (k1, n2) of residues 0-3 in the plane's
   // part of the pair's first row, those of residues 4-7 in the second row.  A line then belongs to one warp
   // from its loads to its last store: no row buffer, no block barrier between the row steps, and the shared
@@ -826,16 +844,18 @@ struct CoopForward {
   }
 
   // Row step 1 of a warp's task: straight from global memory (N2 neighbouring floats per row and lane
-  // group: whole 32-byte sectors), two items in flight per lane, N1-point transform, twiddle, into mid.
+  // group: whole 32-byte sectors), two items in flight per lane (one, for half a task), N1-point transform,
+  // twiddle, into mid.
   static FBF_HD void row_step1(const FftParams& p, const FftGeom& g, char* smem, int lane, int row, int inner0,
-                               int line0, const float2 (&tw)[N1]) {
+                               int line0, const float2 (&tw)[N1], bool half = false) {
     float2* mid = reinterpret_cast<float2*>(smem + g.off_b);
     const long long plane_elems = (long long)p.h * p.w;
     const float* base = p.real_in + (row * p.real_row_stride + inner0 * p.real_inner_stride) * plane_elems;
     const long long tstride = p.real_inner_stride * plane_elems;
     RowLoad r0, r1;
+    r1.slot = -1;
     row_fetch(p, g, base, tstride, inner0, line0, lane, r0);
-    row_fetch(p, g, base, tstride, inner0, line0, lane + 32, r1);
+    if (!half) row_fetch(p, g, base, tstride, inner0, line0, lane + 32, r1);
     row_transform(mid, r0, tw);
     row_transform(mid, r1, tw);
   }

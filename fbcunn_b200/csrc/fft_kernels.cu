@@ -176,15 +176,24 @@ __device__ __forceinline__ int operand_of_tile(const FftBatch<OPS>& b, int& tile
   }
 }
 
-template <int N, int T, int OPS>
-__global__ void __launch_bounds__(coop_threads(N), coop_blocks(N))
+// Whether the warps of a cooperative block take the row lines in halves of a task: where a tile has few of them
+// (filter planes), so that more warps share them, and half a task still fills the lanes in both row steps.
+template <class C>
+__device__ __forceinline__ bool half_tasks(const FftGeom& g, int threads) {
+  constexpr int kHalf = C::L::TASK_LINES / 2;
+  return kHalf * C::N1 >= 32 && kHalf * C::N2 >= 32 && g.lines1 <= (threads >> 5) * kHalf;
+}
+
+// PM: the spectra are plane-major (bins contiguous), else bin-major.
+template <int N, int T, int OPS, bool PM>
+__global__ void __launch_bounds__(coop_shape(N, false, PM).threads, coop_shape(N, false, PM).blocks)
 fft2d_forward_coop_kernel(const __grid_constant__ FftBatch<OPS> b) {
   extern __shared__ __align__(16) char smem[];
   const int tid = threadIdx.x, nth = blockDim.x, lane = tid & 31, warp = tid >> 5;
   const int total = b.tile_end[OPS - 1];
   grid_dependency_wait();
   // persistent blocks: tile w, then w + gridDim.x, ...; the real planes of the next tile are
-  // pulled into L2 while this one is transformed
+  // pulled into L2 while this one is transformed (CoopShape::persistent; else a block has one tile)
   for (int w = blockIdx.x; w < total; w += gridDim.x) {
   int tile = w;
   const int op = operand_of_tile(b, tile);
@@ -205,17 +214,18 @@ fft2d_forward_coop_kernel(const __grid_constant__ FftBatch<OPS> b) {
     }
   }
   using F = CoopForward<N, T>;
-  constexpr int kTask = F::L::TASK_LINES;
   {
+    const bool half = half_tasks<F>(g, nth);
+    const int task = half ? F::L::TASK_LINES / 2 : F::L::TASK_LINES;
     float2 tw[F::N1];  // a lane meets the same n2 in all its items
     F::row_twiddles(lane, tw);
-    for (int line0 = warp * kTask; line0 < g.lines1; line0 += (nth >> 5) * kTask) {
-      F::row_step1(p, g, smem, lane, row, inner0, line0, tw);
+    for (int line0 = warp * task; line0 < g.lines1; line0 += (nth >> 5) * task) {
+      F::row_step1(p, g, smem, lane, row, inner0, line0, tw, half);
       __syncwarp();
       // groups of eight lanes hold the eight residues of one line; mirror residues are
       // neighbours, so one shuffle hands each lane the partner's odd-indexed outputs
 #pragma unroll 1
-      for (int item = lane; item < kTask * F::N1; item += 32) {
+      for (int item = lane; item < task * F::N1; item += 32) {
         float2 u[F::N2], mirror_odd[F::N2 / 2];
         const bool active = F::row_step2_fft(g, smem, line0, item, u);
 #pragma unroll
@@ -231,16 +241,13 @@ fft2d_forward_coop_kernel(const __grid_constant__ FftBatch<OPS> b) {
   __syncthreads();
   CoopForward<N, T>::col_step1(g, smem, tid, nth);
   __syncthreads();
-  if (p.spec_bin == 1 && p.spec_inner == (N / 2 + 1) * N)
-    CoopForward<N, T>::template col_step2<true>(p, g, smem, tid, nth, row, inner0);
-  else
-    CoopForward<N, T>::template col_step2<false>(p, g, smem, tid, nth, row, inner0);
+  CoopForward<N, T>::template col_step2<PM>(p, g, smem, tid, nth, row, inner0);
   __syncthreads();  // the buffers are reused by the next tile
   }
 }
 
-template <int N, int T, int OPS>
-__global__ void __launch_bounds__(coop_threads(N), coop_blocks(N))
+template <int N, int T, int OPS, bool PM>
+__global__ void __launch_bounds__(coop_shape(N, true, PM).threads, coop_shape(N, true, PM).blocks)
 fft2d_inverse_coop_kernel(const __grid_constant__ FftBatch<OPS> b) {
   extern __shared__ __align__(16) char smem[];
   const int tid = threadIdx.x, nth = blockDim.x, lane = tid & 31, warp = tid >> 5;
@@ -259,7 +266,7 @@ fft2d_inverse_coop_kernel(const __grid_constant__ FftBatch<OPS> b) {
   const int tiles_x = b.tiles_x[op];
   const int row = tile / tiles_x;
   const int inner0 = (tile - row * tiles_x) * T;
-  if (p.spec_bin == 1 && tile + step < tiles_x * p.n_rows) {  // plane-major: the next tile's spectra are contiguous
+  if (PM && tile + step < tiles_x * p.n_rows) {  // plane-major: the next tile's spectra are contiguous
     const int wn = tile + step;
     const int rown = wn / tiles_x, innern = (wn - rown * tiles_x) * T;
     const long long plane_bytes = (long long)(N / 2 + 1) * N * 8;
@@ -269,28 +276,26 @@ fft2d_inverse_coop_kernel(const __grid_constant__ FftBatch<OPS> b) {
       for (long long off = (long long)tid * 128; off < plane_bytes; off += (long long)nth * 128) prefetch_l2(src + off);
     }
   }
-  if (p.spec_bin == 1 && p.spec_inner == (N / 2 + 1) * N)
-    CoopInverse<N, T>::template col_step1<true>(p, g, smem, tid, nth, row, inner0);
-  else
-    CoopInverse<N, T>::template col_step1<false>(p, g, smem, tid, nth, row, inner0);
+  CoopInverse<N, T>::template col_step1<PM>(p, g, smem, tid, nth, row, inner0);
   __syncthreads();
   CoopInverse<N, T>::col_step2(g, smem, tid, nth);
   __syncthreads();
   using I = CoopInverse<N, T>;
-  constexpr int kTask = I::L::TASK_LINES;
   {
+    const bool half = half_tasks<I>(g, nth);
+    const int task = half ? I::L::TASK_LINES / 2 : I::L::TASK_LINES;
     float2 tw[I::N1];  // a lane meets the same n2 in all its items
     I::row_twiddles(lane, tw);
-    for (int line0 = warp * kTask; line0 < g.lines1; line0 += (nth >> 5) * kTask) {
+    for (int line0 = warp * task; line0 < g.lines1; line0 += (nth >> 5) * task) {
       float2 v0[I::N1], v1[I::N1];
       const bool on0 = I::row_step1_fft(p, g, smem, line0, lane, v0);
-      const bool on1 = I::row_step1_fft(p, g, smem, line0, lane + 32, v1);
+      const bool on1 = !half && I::row_step1_fft(p, g, smem, line0, lane + 32, v1);
       __syncwarp();
       if (on0) I::row_step1_store(p, g, smem, line0, lane, v0, tw);
       if (on1) I::row_step1_store(p, g, smem, line0, lane + 32, v1, tw);
       __syncwarp();
 #pragma unroll 1
-      for (int item = lane; item < kTask * I::N1; item += 32) I::row_step2(p, g, smem, row, inner0, line0, item);
+      for (int item = lane; item < task * I::N1; item += 32) I::row_step2(p, g, smem, row, inner0, line0, item);
     }
   }
   __syncthreads();  // mid is rewritten by the next tile
@@ -335,10 +340,19 @@ fft1d_inverse_kernel(const __grid_constant__ FftParams p, const __grid_constant_
   Inverse<N, T>::store(p, g, smem, tid, nth, 0, inner0);
 }
 
-// Blocks of a persistent cooperative kernel: as many as are resident at once.
-int persistent_blocks(int N, long long tiles) {
-  const long long resident = (long long)sm_count() * coop_blocks(N);
-  return (int)(tiles < resident ? tiles : resident);
+// Blocks of a cooperative kernel: persistent ones as many as are resident at once.
+long long coop_grid(const CoopShape& shape, long long tiles) {
+  const long long resident = (long long)sm_count() * shape.blocks;
+  return shape.persistent && tiles > resident ? resident : tiles;
+}
+
+template <int N, int T, int OPS, bool PM>
+constexpr auto coop_kernel(bool inverse) {
+  constexpr CoopShape f = coop_shape(N, false, PM), i = coop_shape(N, true, PM);
+  static_assert(f.threads % 32 == 0 && i.threads % 32 == 0, "whole warps");
+  constexpr int blocks = f.blocks > i.blocks ? f.blocks : i.blocks;
+  static_assert(blocks * (N * CoopLayout<N, T>::PITCH2 * 8 + 1024) <= 228 * 1024, "shared memory of an SM");
+  return inverse ? fft2d_inverse_coop_kernel<N, T, OPS, PM> : fft2d_forward_coop_kernel<N, T, OPS, PM>;
 }
 
 // The kernels address the spectrum with 32-bit element offsets.
@@ -354,13 +368,15 @@ cudaError_t run_batch(bool inverse, const FftParams* ops, int count, const RowSu
   long long tiles = 0;
   int smem = 0;
   int mode = kPlanes;
+  const bool plane_major = ops[0].spec_bin == 1;
   for (int i = 0; i < OPS; ++i) {
     if (i < count) {
+      if ((ops[i].spec_bin == 1) != plane_major) return cudaErrorInvalidConfiguration;
       b.p[i] = ops[i];
       if (ops[i].view.nw) mode = kTiles;
       if (ops[i].reference) mode = kReference;
-      b.g[i] = inverse ? inverse_geom(N, T, ops[i].h, ops[i].w)
-                       : forward_geom(N, T, ops[i].h, ops[i].w, ops[i].off_y, ops[i].off_x);
+      b.g[i] = inverse ? inverse_geom(N, T, ops[i].h, ops[i].w, plane_major)
+                       : forward_geom(N, T, ops[i].h, ops[i].w, ops[i].off_y, ops[i].off_x, plane_major);
       b.tiles_x[i] = ((inverse ? ops[i].n_inner : ops[i].kc) + T - 1) / T;
       tiles += (long long)b.tiles_x[i] * ops[i].n_rows;
       if (b.g[i].smem_bytes > smem) smem = b.g[i].smem_bytes;
@@ -376,9 +392,8 @@ cudaError_t run_batch(bool inverse, const FftParams* ops, int count, const RowSu
   void (*kernel)(FftBatch<OPS>);
   long long blocks = tiles;
   if constexpr (N > 32) {
-    kernel = inverse ? fft2d_inverse_coop_kernel<N, T, OPS> : fft2d_forward_coop_kernel<N, T, OPS>;
-    static_assert(coop_blocks(N) * (N * CoopLayout<N, T>::PITCH2 * 8 + 1024) <= 228 * 1024, "shared memory of an SM");
-    blocks = persistent_blocks(N, tiles);
+    kernel = plane_major ? coop_kernel<N, T, OPS, true>(inverse) : coop_kernel<N, T, OPS, false>(inverse);
+    blocks = coop_grid(coop_shape(N, inverse, plane_major), tiles);
   } else {
     if (threads != block_threads<N, T>()) return cudaErrorInvalidConfiguration;
     kernel = inverse ? fft2d_inverse_kernel<N, T, OPS, kPlanes> : fft2d_forward_kernel<N, T, OPS, kPlanes>;

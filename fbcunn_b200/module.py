@@ -63,6 +63,12 @@ def _is_number(x) -> bool:
     return isinstance(x, (int, float)) and not isinstance(x, bool)
 
 
+def own_passes(module, passes) -> bool:
+    """Whether `module` runs the two given functions as its backward passes, so that one call may stand for both."""
+    return (getattr(module.updateGradInput, "__func__", None) is passes[0]
+            and getattr(module.accGradParameters, "__func__", None) is passes[1])
+
+
 class SpatialConvolutionFBFFT:
     """nn.SpatialConvolutionFBFFT(nInputPlane, nOutputPlane, kW, kH, dW, dH, padLeft,
     padUp, memoryReusePolicy, numCudaStreams)."""
@@ -193,11 +199,9 @@ class SpatialConvolutionFBFFT:
 
     def backward(self, input, gradOutput, scale=None):
         """updateGradInput and accGradParameters (fbcunn/SpatialConvolutionFFT.lua:405-416) in one native
-        call, which transforms gradOutput once for both.  A subclass with passes of its own gets them
-        called one after the other."""
-        cls = type(self)
-        if (cls.updateGradInput is not SpatialConvolutionFBFFT.updateGradInput
-                or cls.accGradParameters is not SpatialConvolutionFBFFT.accGradParameters):
+        call, which transforms gradOutput once for both.  Passes that a subclass, the object itself or a
+        patched class brings are called one after the other."""
+        if not own_passes(self, _PASSES):
             self.updateGradInput(input, gradOutput)
             self.accGradParameters(input, gradOutput, scale)
             return self.gradInput
@@ -210,7 +214,7 @@ class SpatialConvolutionFBFFT:
             self.gradInput = torch.empty_like(input)
         capi.check(capi.lib().fbfftconv_backward(
             h, input.data_ptr(), gradOutput.data_ptr(), self.weight.data_ptr(), self.gradInput.data_ptr(),
-            self.gradWeight.data_ptr(), self.gradBias.data_ptr(), 1.0 if scale is None else float(scale),
+            self.gradWeight.data_ptr(), _ptr(self.gradBias), 1.0 if scale is None else float(scale),
             _stream(self.device)))
         return self.gradInput
 
@@ -326,6 +330,10 @@ class SpatialConvolutionFBFFT:
             self.cleanupBuffers()
         except Exception:
             pass
+
+
+# the backward passes as they are defined above, whatever becomes of the class attributes
+_PASSES = (SpatialConvolutionFBFFT.updateGradInput, SpatialConvolutionFBFFT.accGradParameters)
 
 
 class SpatialConvolutionFBFFTGemm(SpatialConvolutionFBFFT):

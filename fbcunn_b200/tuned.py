@@ -20,7 +20,7 @@ from typing import Callable, List, Optional, Tuple
 import torch
 
 from . import capi
-from .module import SpatialConvolutionFBFFT, memoryReuseAll, memoryReuseNone
+from .module import SpatialConvolutionFBFFT, memoryReuseAll, memoryReuseNone, own_passes
 from .tiled import SpatialConvolutionFFTTiled
 
 Candidate = Tuple[str, Callable[[], SpatialConvolutionFBFFT]]
@@ -168,6 +168,10 @@ class SpatialConvolution:
         return self.updateOutput(input)
 
     def backward(self, input, gradOutput, scale=None):
+        if not own_passes(self, _PASSES):
+            self.updateGradInput(input, gradOutput)
+            self.accGradParameters(input, gradOutput, scale)
+            return self.gradInput
         assert self.bestModuleInst is not None, "updateOutput runs first (it tunes)"
         assert not self.inferenceOnly, "module was built for inference only"
         self.gradInput = self.bestModuleInst.backward(input, gradOutput, scale)
@@ -181,3 +185,6 @@ class SpatialConvolution:
         if self.bestModuleInst is not None:
             self.bestModuleInst.cleanupBuffers()
 
+
+# the backward passes as they are defined above, whatever becomes of the class attributes
+_PASSES = (SpatialConvolution.updateGradInput, SpatialConvolution.accGradParameters)

@@ -694,30 +694,30 @@ Operand grad_output_operand(const fbfftconv_handle* h, int stage, const float* g
   return op;
 }
 
-// Whether transforms run as one launch.  Up to 32 points always: one wave fewer, and no launch gap.  The
-// persistent kernels of the larger sizes only where some operand has too few tiles to fill the GPU (four per
-// SM): their single-operand form is a little faster per plane.
-bool merge_transforms(int N, const FftParams* p, int count) {
-  if (count < 2 || count > kMaxFftOps) return false;
-  if (N <= 32) return true;
-  for (int i = 0; i < count; ++i) {
-    const int T = fft_tile(N);
-    if ((long long)p[i].n_rows * ((p[i].n_inner + T - 1) / T) < 4LL * sm_count()) return true;
-  }
-  return false;
+// Whether a transform shares a launch with the pass's other ones.  Up to 32 points always: one wave fewer, and no
+// launch gap.  The cooperative kernels of the larger sizes only where it has too few tiles to fill the GPU (four
+// per SM): small transforms beside each other fill it better, while a large one loses in the kernel that looks its
+// operand up.  updateOutput / backward, us, sharing up to 0, 4 and 16 tiles per SM: 16 x 3 -> 96 planes of 128 x 128 (11 x 11 filters) 118 / 166, 110 / 154, 110 / 151;
+// 8 x 32 -> 64 of 64 x 64 (9 x 9) 63 / 130, 56 / 116, 56 / 116; 32 x 16 -> 64 of 100 x 100 (7 x 7) 349 / 678,
+// 341 / 678, 355 / 693.  (Every operand shared wherever one is small: 4 x 64 -> 128
+// of 128 x 128 with 5 x 5 filters 1010 / 1756 against 796 / 1544.)
+bool shares_launch(int N, const FftParams& p) {
+  const int T = fft_tile(N);
+  return N <= 32 || (long long)p.n_rows * ((p.n_inner + T - 1) / T) < 4LL * sm_count();
 }
 
 int forward_transforms(fbfftconv_handle* h, int pass, const Operand* ops, int count, cudaStream_t s) {
-  FftParams p[kMaxFftOps];
-  for (int i = 0; i < count; ++i) p[i] = ops[i].p;
-  if (!h->profiling && merge_transforms(h->N, p, count)) {
-    FBF_CUDA(launch_forward(p, count, h->N, s));
-    return FBFFTCONV_OK;
-  }
+  FftParams shared[kMaxFftOps];
+  int n_shared = 0;
   for (int i = 0; i < count; ++i) {
+    if (!h->profiling && shares_launch(h->N, ops[i].p)) {
+      shared[n_shared++] = ops[i].p;
+      continue;
+    }
     StageTimer t(h, pass, ops[i].stage, s);
-    FBF_CUDA(launch_forward(&p[i], 1, h->N, s));
+    FBF_CUDA(launch_forward(&ops[i].p, 1, h->N, s));
   }
+  if (n_shared) FBF_CUDA(launch_forward(shared, n_shared, h->N, s));
   return FBFFTCONV_OK;
 }
 
@@ -1132,7 +1132,7 @@ int fbfftconv_backward(fbfftconv_handle* h, const float* input, const float* gra
                                            d.kernel_h, d.kernel_w, 0, 0, accumulate, h->plane_major ? 2 : 0, h->N)};
   RowSum sum{};
   if (grad_bias) sum = bias_sum(h, grad_bias, scale, accumulate);
-  if (merge_transforms(h->N, inv, 2)) {
+  if (shares_launch(h->N, inv[0]) && shares_launch(h->N, inv[1])) {
     FBF_CUDA(launch_inverse(inv, 2, &sum, h->N, s));
   } else {
     FBF_CUDA(launch_inverse(&inv[0], 1, nullptr, h->N, s));

@@ -160,8 +160,8 @@ __device__ __forceinline__ void prefetch_l2(const void* p) {
   asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }
 
-// The persistent kernels look the operand up per tile (only small layers and the small operands of larger
-// ones reach the merged form): `tile` becomes the tile's number inside the operand.
+// The cooperative kernels look the operand up per tile (only operands that do not fill the GPU by themselves reach
+// the merged form): `tile` becomes the tile's number inside the operand.
 template <int OPS>
 __device__ __forceinline__ int operand_of_tile(const FftBatch<OPS>& b, int& tile) {
   if constexpr (OPS == 1) {

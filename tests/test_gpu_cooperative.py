@@ -8,7 +8,8 @@ import numpy as np
 import pytest
 import torch
 
-from fbcunn_b200 import capi
+import oracle
+from fbcunn_b200 import SpatialConvolutionFBFFT, capi
 from oracle import spectral
 
 pytestmark = pytest.mark.gpu
@@ -50,3 +51,25 @@ def test_forward_and_inverse(n, shape, plane_major):
                                            stream))
     want = n * n * x.astype(np.float64) + bias.cpu().numpy()[None, :, None, None]
     assert np.abs(back.cpu().numpy() - want).max() <= TOL * np.abs(want).max()
+
+
+# layers with one transform that fills the GPU (four tiles per SM) beside ones that do not: 64 points bin-major, 128
+# points plane-major, 128 points bin-major
+@pytest.mark.parametrize("s", [oracle.Shape(300, 8, 2, 40, 38, 3, 3), oracle.Shape(200, 3, 1, 70, 66, 3, 2, 1, 0),
+                               oracle.Shape(100, 6, 1, 66, 70, 2, 3)], ids=lambda s: "x".join(map(str, (s.B, s.P, s.iH))))
+def test_large_and_small_operands(s):
+    def rel(a, ref):
+        return float(np.abs(a.cpu().numpy() - ref).max() / np.abs(ref).max())
+
+    rng = np.random.default_rng(s.B)
+    x = rng.standard_normal((s.B, s.P, s.iH, s.iW)).astype(np.float32)
+    go = rng.standard_normal((s.B, s.F, s.oH, s.oW)).astype(np.float32)
+    m = SpatialConvolutionFBFFT(s.P, s.F, s.kW, s.kH, 1, 1, s.padW, s.padH)
+    w, b = m.weight.cpu().numpy(), m.bias.cpu().numpy()
+    dx, dgo = torch.from_numpy(x).cuda(), torch.from_numpy(go).cuda()
+    before = capi.kernel_launches()
+    assert rel(m.forward(dx), oracle.update_output(s, x, w, b)) <= 1e-4
+    assert capi.kernel_launches() - before == 4  # the large transform has a launch of its own
+    assert rel(m.backward(dx, dgo), oracle.update_grad_input(s, go, w)) <= 1e-4
+    assert rel(m.gradWeight, oracle.acc_grad_weight(s, x, go, 1.0)) <= 1e-4
+    assert rel(m.gradBias, oracle.acc_grad_bias(s, go, 1.0)) <= 1e-4

@@ -29,6 +29,7 @@ REUSE_INPUT = 16
 REUSE_OUTPUT = 32
 REUSE_WEIGHT = 64
 EXCHANGE_NCCL = 128
+MIN_WORKSPACE = 256
 
 
 class Desc(ctypes.Structure):

@@ -132,6 +132,8 @@ struct fbfftconv_handle {
   bool plane_major = false;  // <= 4 input planes at a cooperative transform size: see contract_stream.cu
   // frequency buffers, each sized for the largest use among the three passes
   size_t bytes_in, bytes_out, bytes_w, bytes_small, bytes_gi, bytes_total;
+  size_t spare_gi = 0;  // gradInput buffer that the passes can do without (part of bytes_total, not of bytes_min)
+  size_t bytes_min;
   // spectrum reuse (plane-major layers only): which tensor's forward spectrum a buffer holds
   bool have_input_spec = false, have_grad_output_spec = false, have_weight_spec = false;
   // set by a backward call between its two passes: the second one is handed the gradOutput whose spectrum
@@ -184,14 +186,27 @@ namespace {
 size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 
 // Up to this size the gradInput spectrum gets a buffer of its own even where no flag asks for it, so that a
-// backward call can transform its three operands in one launch and invert its two products in another: that
-// saves launches, which larger layers do not feel.
+// backward call can transform its three operands in one launch and invert its two products in another, two
+// launches less.  backward without / with it, us (size of the input spectrum): 64 x 16 -> 32 planes of 16 x 16
+// 27.4 / 20.4 (1.2 MB), 16 x 16 -> 16 of 32 x 32 33.1 / 27.2 (1.1 MB), 128 x 64 -> 64 of 16 x 16 39.0 / 35.1
+// (9.4 MB); beyond the line 128 x 128 -> 128 of 16 x 16 62.9 / 60.7 (18.9 MB), 64 x 64 -> 64 of 32 x 32 74.3 / 73.0
+// (17.8 MB), 128 x 384 -> 384 of 13 x 13 315 / 316 (57 MB): not worth the memory there.
 constexpr size_t kOwnGradInputBytes = size_t(16) << 20;
+
+// With the gradInput buffer that the passes can do without, or without it.
+void take_spare(fbfftconv_handle* h, bool take) {
+  if (h->spare_gi) h->bytes_gi = take ? h->spare_gi : 0;
+}
 
 int ensure_workspace(fbfftconv_handle* h) {
   if (h->ws) return FBFFTCONV_OK;
   void* p = nullptr;
   cudaError_t e = cudaMalloc(&p, h->bytes_total);
+  take_spare(h, e != cudaErrorMemoryAllocation);
+  if (e == cudaErrorMemoryAllocation && h->spare_gi) {
+    cudaGetLastError();
+    e = cudaMalloc(&p, h->bytes_min);
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(e == cudaErrorMemoryAllocation ? FBFFTCONV_ERR_NOMEM : FBFFTCONV_ERR_CUDA,
@@ -600,8 +615,11 @@ int fbfftconv_create(const fbfftconv_desc* desc, fbfftconv_handle** out) {
   h->bytes_small = align256((B * F + F) * sizeof(float));
   // local gradWeight + gradBias where they are summed or gathered across ranks in the spatial domain
   h->bytes_small += 2 * align256((F * P * d.kernel_h * d.kernel_w + F) * sizeof(float));  // vec_in, vec_out
-  h->bytes_gi = (d.flags & FBFFTCONV_REUSE_INPUT) || h->bytes_in <= kOwnGradInputBytes ? h->bytes_in : 0;
-  h->bytes_total = h->bytes_in + h->bytes_out + h->bytes_w + h->bytes_small + h->bytes_gi;
+  h->bytes_gi = (d.flags & FBFFTCONV_REUSE_INPUT) ? h->bytes_in : 0;
+  h->bytes_min = h->bytes_in + h->bytes_out + h->bytes_w + h->bytes_small + h->bytes_gi;
+  if (!h->bytes_gi && h->bytes_in <= kOwnGradInputBytes && !(d.flags & FBFFTCONV_MIN_WORKSPACE)) h->spare_gi = h->bytes_in;
+  h->bytes_total = h->bytes_min + h->spare_gi;
+  take_spare(h, true);
   *out = h;
   return FBFFTCONV_OK;
 }
@@ -636,9 +654,10 @@ size_t fbfftconv_workspace_bytes(const fbfftconv_handle* h) { return h ? h->byte
 
 int fbfftconv_set_workspace(fbfftconv_handle* h, void* device_ptr, size_t bytes) {
   if (!h) return fail(FBFFTCONV_ERR_INVALID_ARGUMENT, "null handle");
-  if (!device_ptr || bytes < h->bytes_total || (reinterpret_cast<uintptr_t>(device_ptr) & 255))
+  if (!device_ptr || bytes < h->bytes_min || (reinterpret_cast<uintptr_t>(device_ptr) & 255))
     return fail(FBFFTCONV_ERR_INVALID_ARGUMENT,
-                "workspace must be 256-byte aligned and hold %zu bytes", h->bytes_total);
+                "workspace must be 256-byte aligned and hold %zu bytes", h->bytes_min);
+  take_spare(h, bytes >= h->bytes_total);
   if (h->ws && h->ws_owned) {
     DeviceGuard g;
     g.enter(h->device);
@@ -697,10 +716,10 @@ Operand grad_output_operand(const fbfftconv_handle* h, int stage, const float* g
 // Whether a transform shares a launch with the pass's other ones.  Up to 32 points always: one wave fewer, and no
 // launch gap.  The cooperative kernels of the larger sizes only where it has too few tiles to fill the GPU (four
 // per SM): small transforms beside each other fill it better, while a large one loses in the kernel that looks its
-// operand up.  updateOutput / backward, us, sharing up to 0, 4 and 16 tiles per SM: 16 x 3 -> 96 planes of 128 x 128 (11 x 11 filters) 118 / 166, 110 / 154, 110 / 151;
-// 8 x 32 -> 64 of 64 x 64 (9 x 9) 63 / 130, 56 / 116, 56 / 116; 32 x 16 -> 64 of 100 x 100 (7 x 7) 349 / 678,
-// 341 / 678, 355 / 693.  (Every operand shared wherever one is small: 4 x 64 -> 128
-// of 128 x 128 with 5 x 5 filters 1010 / 1756 against 796 / 1544.)
+// operand up.  updateOutput / backward, us, sharing up to 0, 4 and 16 tiles per SM: 16 x 3 -> 96 planes of
+// 128 x 128 (11 x 11 filters) 118 / 166, 110 / 154, 110 / 151; 8 x 32 -> 64 of 64 x 64 (9 x 9) 63 / 130, 56 / 116,
+// 56 / 116; 32 x 16 -> 64 of 100 x 100 (7 x 7) 349 / 678, 341 / 678, 355 / 693.  (Every operand shared wherever one
+// is small: 4 x 64 -> 128 of 128 x 128 with 5 x 5 filters 1010 / 1756 against 796 / 1544.)
 bool shares_launch(int N, const FftParams& p) {
   const int T = fft_tile(N);
   return N <= 32 || (long long)p.n_rows * ((p.n_inner + T - 1) / T) < 4LL * sm_count();

@@ -75,7 +75,8 @@ class SpatialConvolutionFBFFT:
 
     def __init__(self, nInputPlane, nOutputPlane, kW, kH, dW=1, dH=1, padLeft=0, padUp=0,
                  memoryReusePolicy=None, numCudaStreams=None, *, device="cuda", accumulate=False,
-                 contraction: str = "auto", allreduce: str = "spectrum", exchange: str = "auto"):
+                 contraction: str = "auto", allreduce: str = "spectrum", exchange: str = "auto",
+                 min_workspace: bool = False):
         for v in (nInputPlane, nOutputPlane, kW, kH, dW, dH, padLeft, padUp):
             assert _is_number(v), "constructor arguments must be numbers"
         assert memoryReusePolicy is None or isinstance(memoryReusePolicy, (str, list, tuple))
@@ -115,6 +116,8 @@ class SpatialConvolutionFBFFT:
         # who carries that sum: the library's kernels over peer memory where they apply ("auto"), or NCCL only
         assert exchange in ("auto", "nccl")
         self._exchange = exchange
+        # no more scratch than the passes need (FBFFTCONV_MIN_WORKSPACE)
+        self._min_workspace = bool(min_workspace)
         shape_w = (self.nOutputPlane, self.nInputPlane, self.kH, self.kW)
         self.weight = torch.empty(shape_w, dtype=torch.float32, device=self.device)
         self.bias = torch.empty(self.nOutputPlane, dtype=torch.float32, device=self.device)
@@ -299,6 +302,7 @@ class SpatialConvolutionFBFFT:
                 (capi.BIN_MAJOR_ONLY if self._contraction == "bin_major" else 0) | \
                 (capi.ALLREDUCE_SPATIAL if self._allreduce == "spatial" else 0) | \
                 (capi.EXCHANGE_NCCL if self._exchange == "nccl" else 0) | \
+                (capi.MIN_WORKSPACE if self._min_workspace else 0) | \
                 (capi.REUSE_INPUT if memoryReuseInput in self.memoryReusePolicy else 0) | \
                 (capi.REUSE_OUTPUT if memoryReuseOutput in self.memoryReusePolicy else 0) | \
                 (capi.REUSE_WEIGHT if memoryReuseWeight in self.memoryReusePolicy else 0)

@@ -98,7 +98,8 @@ class SpatialConvolution:
         self.maximalMemoryOverhead = maximalMemoryOverhead
         self.inferenceOnly = bool(inferenceOnly)
         self.device = device
-        self._kw = dict(kw, device=device)
+        # under a memory limit the candidates take no more scratch than they need
+        self._kw = dict({"min_workspace": maximalMemoryOverhead is not None}, **kw, device=device)
         self._timer = timer or time_module
         self.bestModuleInst = None
         self.timings = {}

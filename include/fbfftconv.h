@@ -75,7 +75,9 @@ enum {
   FBFFTCONV_REUSE_WEIGHT = 64,
   /* with a communicator attached, keep the whole weight-gradient exchange on NCCL instead of the
    * sums over peer memory described at fbfftconv_comm_init (must be the same on every rank) */
-  FBFFTCONV_EXCHANGE_NCCL = 128
+  FBFFTCONV_EXCHANGE_NCCL = 128,
+  /* no more scratch than the passes need: see fbfftconv_workspace_bytes */
+  FBFFTCONV_MIN_WORKSPACE = 256
 };
 
 /* Constructor arguments of nn.SpatialConvolutionFBFFT
@@ -106,10 +108,13 @@ int fbfftconv_destroy(fbfftconv_handle* h);
 /* Transform size N chosen for the layer (fbcunn/SpatialConvolutionFFT.lua:875-882). */
 int fbfftconv_fft_size(const fbfftconv_handle* h);
 /* Bytes of device scratch the three passes need (the reference's inputBuffer /
- * outputBuffer / weightBuffer, fbcunn/SpatialConvolutionFFT.lua:652-688). */
+ * outputBuffer / weightBuffer, fbcunn/SpatialConvolutionFFT.lua:652-688).  For layers whose input spectrum is at
+ * most 16 MB they include a buffer of its own for the gradInput spectrum, of that size, which saves
+ * fbfftconv_backward launches; the passes do without it where FBFFTCONV_MIN_WORKSPACE asks for that, where the
+ * caller's block is smaller by that much, and where cudaMalloc cannot give it. */
 size_t fbfftconv_workspace_bytes(const fbfftconv_handle* h);
 /* Optional: hand the library a caller-owned scratch block of at least
- * fbfftconv_workspace_bytes(); otherwise it is allocated with cudaMalloc on the
+ * fbfftconv_workspace_bytes() (or what that is with FBFFTCONV_MIN_WORKSPACE); otherwise it is allocated with cudaMalloc on the
  * first pass and freed by fbfftconv_destroy. */
 int fbfftconv_set_workspace(fbfftconv_handle* h, void* device_ptr, size_t bytes);
 

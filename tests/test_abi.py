@@ -100,6 +100,29 @@ def test_workspace_accounting(lib):
     lib.fbfftconv_destroy(h)
 
 
+def test_workspace_without_the_spare_buffer(lib):
+    """A layer whose passes use a gradInput buffer where they have one also takes a block without it; a layer that
+    needs the buffer (reused input spectrum) does not, and a large layer has none."""
+    def sizes(**kw):
+        out = []
+        for flags in (0, capi.MIN_WORKSPACE):
+            rc, h = _create(lib, **{**kw, "flags": kw.get("flags", 0) | flags})
+            assert rc == capi.OK
+            out.append((h, lib.fbfftconv_workspace_bytes(h)))
+        return out
+
+    block = ctypes.c_void_p(1 << 20)  # 256-byte aligned, never touched here
+    for kw, spare in [(dict(batch=16, n_input_plane=16, input_h=30, input_w=30), 17 * 32 * 16 * 16 * 8),
+                      (dict(flags=capi.REUSE_INPUT), 0),
+                      (dict(batch=128, n_input_plane=384, n_output_plane=384, input_h=13, input_w=13), 0)]:
+        (h, full), (h_min, least) = sizes(**kw)
+        assert full - least == spare
+        for handle in (h, h_min):
+            assert lib.fbfftconv_set_workspace(handle, block, least - 1) == capi.ERR_INVALID_ARGUMENT
+            assert lib.fbfftconv_set_workspace(handle, block, least) == capi.OK
+            assert lib.fbfftconv_destroy(handle) == capi.OK
+
+
 def test_substeps_reject_bad_arguments(lib):
     assert lib.fbfftconv_fft2d(None, None, 1, 1, 4, 4, 8, 0, 0, 0, None) == capi.ERR_INVALID_ARGUMENT
     one = ctypes.c_void_p(16)

@@ -6,7 +6,7 @@ import pytest
 import torch
 
 import oracle
-from fbcunn_b200 import SpatialConvolutionFBFFT
+from fbcunn_b200 import SpatialConvolutionFBFFT, capi
 
 pytestmark = pytest.mark.gpu
 PASS_TOL = 1e-4
@@ -56,3 +56,29 @@ def test_backward_matches_the_oracle(s, reuse):
     b = m2.updateGradInput(dx, dgo), (m2.accGradParameters(dx, dgo), m2.gradWeight)[1], m2.gradBias
     for p, q in zip(a, b):
         assert float((p - q).abs().max()) <= 2e-6 * float(q.abs().max())
+
+
+@pytest.mark.parametrize("spare", [False, True])
+def test_backward_in_a_block_of_the_callers(spare):
+    """The scratch block handed in, with and without room for the gradInput spectrum's own buffer: nothing is written
+    behind it and the same gradients come out."""
+    s = SHAPES[2]
+    rng = np.random.default_rng(3)
+    x = rng.standard_normal((s.B, s.P, s.iH, s.iW)).astype(np.float32)
+    go = rng.standard_normal((s.B, s.F, s.oH, s.oW)).astype(np.float32)
+    m = SpatialConvolutionFBFFT(s.P, s.F, s.kW, s.kH, 1, 1, s.padW, s.padH)
+    least = SpatialConvolutionFBFFT(s.P, s.F, s.kW, s.kH, 1, 1, s.padW, s.padH, min_workspace=True)
+    dx, dgo = torch.from_numpy(x).cuda(), torch.from_numpy(go).cuda()
+    lib = capi.lib()
+    full, need = (lib.fbfftconv_workspace_bytes(layer._prepare(dx)) for layer in (m, least))
+    assert need < full
+    size = full if spare else full - 1
+    block = torch.full((full + 512,), 77, dtype=torch.uint8, device="cuda")
+    first = -block.data_ptr() % 256
+    capi.check(lib.fbfftconv_set_workspace(m._handle, block.data_ptr() + first, size))
+    got = m.backward(dx, dgo)
+    assert _rel(got.cpu().numpy(), oracle.update_grad_input(s, go, m.weight.cpu().numpy())) <= PASS_TOL
+    assert _rel(m.gradWeight.cpu().numpy(), oracle.acc_grad_weight(s, x, go, 1.0)) <= PASS_TOL
+    assert _rel(m.gradBias.cpu().numpy(), oracle.acc_grad_bias(s, go, 1.0)) <= PASS_TOL
+    assert bool((block[first + (full if spare else need):] == 77).all())
+    m.cleanupBuffers()

@@ -5,7 +5,7 @@ import pytest
 import torch
 
 import oracle
-from fbcunn_b200 import SpatialConvolution
+from fbcunn_b200 import SpatialConvolution, capi
 from fbcunn_b200.tuned import candidate_list
 
 
@@ -54,6 +54,17 @@ def test_fastest_candidate_within_the_memory_limit_wins():
     assert m.bestModuleInst.weight is m.weight and m.bestModuleInst.gradWeight is m.gradWeight
     with pytest.raises(ValueError):
         SpatialConvolution(4, 4, 3, 3, 2, 2, device="cpu")
+
+
+def test_a_memory_limit_buys_no_spare_buffer():
+    def timer(inst, x, go, scale, inference_only):
+        flags.append(inst._flags() & capi.MIN_WORKSPACE)
+        return [1.0, 1.0, 1.0], 10
+
+    for limit in (None, 500):
+        flags = []
+        SpatialConvolution(4, 4, 3, 3, 1, 1, 1, 1, limit, device="cpu", timer=timer)._tune(torch.zeros(2, 4, 40, 40))
+        assert flags == [capi.MIN_WORKSPACE if limit else 0] * 6
 
 
 @pytest.mark.gpu

@@ -226,9 +226,8 @@ cudaError_t launch_stream_reduce(const float2* x, const float2* y, float2* z, in
     e = conj_x ? launch(stream_reduce_kernel<2, true, 128>) : launch(stream_reduce_kernel<2, false, 128>);
   else
     e = conj_x ? launch(stream_reduce_kernel<1, true, 128>) : launch(stream_reduce_kernel<1, false, 128>);
-  if (e != cudaSuccess) return e;
-  count_launch();
-  return cudaGetLastError();
+  if (e == cudaSuccess) count_launch();
+  return e;
 }
 
 }  // namespace fbfft

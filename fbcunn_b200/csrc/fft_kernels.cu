@@ -32,11 +32,17 @@ cudaError_t ensure_dynamic_smem(const void* kernel, int bytes) {
     if (e.kernel == kernel && e.device == dev) {
       if (e.bytes >= bytes) return cudaSuccess;
       cudaError_t r = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-      if (r == cudaSuccess) e.bytes = bytes;
+      if (r == cudaSuccess)
+        e.bytes = bytes;
+      else
+        cudaGetLastError();
       return r;
     }
   cudaError_t r = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (r == cudaSuccess) seen.push_back(Entry{kernel, dev, bytes});
+  if (r == cudaSuccess)
+    seen.push_back(Entry{kernel, dev, bytes});
+  else
+    cudaGetLastError();
   return r;
 }
 

@@ -47,7 +47,9 @@ cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, int threads, 
   attr.val.programmaticStreamSerializationAllowed = 1;
   config.attrs = &attr;
   config.numAttrs = 1;
-  return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+  if (e != cudaSuccess) cudaGetLastError();  // returned here; the next launch must not report it again
+  return e;
 }
 
 // ---- transforms ------------------------------------------------------------------------------

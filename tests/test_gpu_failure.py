@@ -93,3 +93,17 @@ def test_host_and_foreign_pointers_are_refused():
     # the module still works afterwards
     m.updateOutput(x)
     torch.cuda.synchronize()
+
+
+def test_a_refused_launch_is_reported_once():
+    """A grid beyond the launch limits (65536 row tiles) is refused by the CUDA runtime before anything runs; the
+    next call, whose launch is fine, does not report it."""
+    lib = capi.lib()
+    t = torch.zeros(1024, device="cuda")
+    p = ctypes.c_void_p(t.data_ptr())
+    rc = lib.fbfftconv_transpose_mm(p, p, p, 1, 64 * 65536, 8, 4, ctypes.c_float(1.0), 0, 0, 1, _stream())
+    assert rc == capi.ERR_CUDA
+    bias, out = torch.ones(2, device="cuda"), torch.zeros(1, 2, 3, 3, device="cuda")
+    capi.check(lib.fbfftconv_update_output_bias(ctypes.c_void_p(out.data_ptr()), ctypes.c_void_p(bias.data_ptr()),
+                                                1, 2, 3, 3, _stream()))
+    assert bool((out == 1).all())

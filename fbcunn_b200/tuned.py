@@ -47,30 +47,27 @@ def candidate_list(nInputPlane, nOutputPlane, kW, kH, padLeft, padUp, iH, iW, **
 
 def time_module(m, input, gradOutput, scale, inference_only, iters=3):
     """Milliseconds per (updateOutput, updateGradInput, accGradParameters), CUDA events on the
-    current stream, after one untimed round; and the bytes of device memory the module took."""
+    current stream, after one untimed round; and the bytes of device memory the module took.
+    accGradParameters counts as what it adds to the other two in a training step of updateOutput and
+    `backward`, where the passes may share work: the three add up to that step."""
     torch.cuda.synchronize()
     before = torch.cuda.memory_allocated()
-
-    def run(which):
-        if which == 0:
-            m.updateOutput(input)
-        elif which == 1:
-            m.updateGradInput(input, gradOutput)
-        else:
-            m.accGradParameters(input, gradOutput, scale)
-
-    passes = (0,) if inference_only else (0, 1, 2)
-    times = [0.0, 0.0, 0.0]
-    for which in passes:
-        run(which)
-    for which in passes:
+    calls = [lambda: m.updateOutput(input)]
+    if not inference_only:
+        calls += [lambda: m.updateGradInput(input, gradOutput),
+                  lambda: (m.updateOutput(input), m.backward(input, gradOutput, scale))]
+    times = []
+    for call in calls:
+        call()
+    for call in calls:
         start, stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         start.record()
         for _ in range(iters):
-            run(which)
+            call()
         stop.record()
         stop.synchronize()
-        times[which] = start.elapsed_time(stop) / iters
+        times.append(start.elapsed_time(stop) / iters)
+    times = [times[0], 0.0, 0.0] if inference_only else [times[0], times[1], max(0.0, times[2] - times[0] - times[1])]
     # device memory the library allocated itself (torch does not see it)
     native = 0
     if getattr(m, "_tiled", None) is not None:

@@ -6,7 +6,7 @@ import torch
 
 import oracle
 from fbcunn_b200 import SpatialConvolution, capi
-from fbcunn_b200.tuned import candidate_list
+from fbcunn_b200.tuned import candidate_list, time_module
 
 
 def _labels(*a):
@@ -65,6 +65,42 @@ def test_a_memory_limit_buys_no_spare_buffer():
         flags = []
         SpatialConvolution(4, 4, 3, 3, 1, 1, 1, 1, limit, device="cpu", timer=timer)._tune(torch.zeros(2, 4, 40, 40))
         assert flags == [capi.MIN_WORKSPACE if limit else 0] * 6
+
+
+def test_candidates_are_timed_as_a_step_runs_them(monkeypatch):
+    """By updateOutput and backward; a clock that the calls advance stands in for the GPU."""
+    clock = [0.0]
+
+    class Event:
+        def __init__(self, enable_timing):
+            pass
+
+        def record(self):
+            self.at = clock[0]
+
+        def synchronize(self):
+            pass
+
+        def elapsed_time(self, other):
+            return other.at - self.at
+
+    class Layer:
+        def updateOutput(self, x):
+            clock[0] += 3
+
+        def updateGradInput(self, x, go):
+            clock[0] += 4
+
+        def accGradParameters(self, x, go, scale):
+            clock[0] += 5
+
+        def backward(self, x, go, scale):
+            clock[0] += 7
+
+    for name, fake in (("Event", Event), ("synchronize", lambda: None), ("memory_allocated", lambda: 0)):
+        monkeypatch.setattr(torch.cuda, name, fake)
+    assert time_module(Layer(), None, None, 0.5, False) == ([3.0, 4.0, 3.0], 0)
+    assert time_module(Layer(), None, None, 0.5, True) == ([3.0, 0.0, 0.0], 0)
 
 
 @pytest.mark.gpu

@@ -773,6 +773,12 @@ struct CoopLayout {
   static FBF_HD int slot_in_half(int k1) { return (k1 & 3) * (N2 + 1); }
   // Lines that a warp takes at a time: two items of the first row step per lane.
   static constexpr int TASK_LINES = 64 / N2;
+  // Half of that where a tile has few lines (filter planes), so that more warps share them, and half a task still
+  // fills the lanes in both row steps (64 points).
+  static FBF_HD bool half_tasks(const FftGeom& g, int threads) {
+    constexpr int kHalf = TASK_LINES / 2;
+    return kHalf * N1 >= 32 && kHalf * N2 >= 32 && g.lines1 <= (threads >> 5) * kHalf;
+  }
 };
 
 // Order of the residues k1 inside a group of eight neighbouring lanes: residues that

@@ -182,14 +182,6 @@ __device__ __forceinline__ int operand_of_tile(const FftBatch<OPS>& b, int& tile
   }
 }
 
-// Whether the warps of a cooperative block take the row lines in halves of a task: where a tile has few of them
-// (filter planes), so that more warps share them, and half a task still fills the lanes in both row steps.
-template <class C>
-__device__ __forceinline__ bool half_tasks(const FftGeom& g, int threads) {
-  constexpr int kHalf = C::L::TASK_LINES / 2;
-  return kHalf * C::N1 >= 32 && kHalf * C::N2 >= 32 && g.lines1 <= (threads >> 5) * kHalf;
-}
-
 // PM: the spectra are plane-major (bins contiguous), else bin-major.
 template <int N, int T, int OPS, bool PM>
 __global__ void __launch_bounds__(coop_shape(N, false, PM).threads, coop_shape(N, false, PM).blocks)
@@ -221,7 +213,7 @@ fft2d_forward_coop_kernel(const __grid_constant__ FftBatch<OPS> b) {
   }
   using F = CoopForward<N, T>;
   {
-    const bool half = half_tasks<F>(g, nth);
+    const bool half = F::L::half_tasks(g, nth);
     const int task = half ? F::L::TASK_LINES / 2 : F::L::TASK_LINES;
     float2 tw[F::N1];  // a lane meets the same n2 in all its items
     F::row_twiddles(lane, tw);
@@ -288,7 +280,7 @@ fft2d_inverse_coop_kernel(const __grid_constant__ FftBatch<OPS> b) {
   __syncthreads();
   using I = CoopInverse<N, T>;
   {
-    const bool half = half_tasks<I>(g, nth);
+    const bool half = I::L::half_tasks(g, nth);
     const int task = half ? I::L::TASK_LINES / 2 : I::L::TASK_LINES;
     float2 tw[I::N1];  // a lane meets the same n2 in all its items
     I::row_twiddles(lane, tw);

@@ -27,14 +27,16 @@ void run_forward(const FftParams& p) {
       std::memset(smem.data(), 0xFF, smem.size());
       if constexpr (N > 32) {
         using F = CoopForward<N, T>;
-        constexpr int N1 = F::N1, N2 = F::N2, kTask = F::L::TASK_LINES;
-        for (int line0 = 0; line0 < g.lines1; line0 += kTask) {  // a warp's task: 32 lanes, in rounds
+        constexpr int N1 = F::N1, N2 = F::N2;
+        const bool half = F::L::half_tasks(g, nth);
+        const int task = half ? F::L::TASK_LINES / 2 : F::L::TASK_LINES;
+        for (int line0 = 0; line0 < g.lines1; line0 += task) {  // a warp's task: 32 lanes, in rounds
           for (int lane = 0; lane < 32; ++lane) {
             float2 tw[N1];
             F::row_twiddles(lane, tw);
-            F::row_step1(p, g, smem.data(), lane, row, inner0, line0, tw);
+            F::row_step1(p, g, smem.data(), lane, row, inner0, line0, tw, half);
           }
-          for (int first = 0; first < kTask * N1; first += 32) {
+          for (int first = 0; first < task * N1; first += 32) {
             // the device exchanges the transforms of mirror residues by a lane shuffle
             std::vector<float2> all(static_cast<size_t>(32) * N2, make_float2(NAN, NAN));
             bool active[32];
@@ -60,9 +62,15 @@ void run_forward(const FftParams& p) {
             CoopForward<N, T>::template col_step2<false>(p, g, smem.data(), tid, nth, row, inner0);
       } else {
         for (int tid = 0; tid < g.threads; ++tid)
-          Forward<N, T>::template load<kTiles>(p, g, smem.data(), tid, g.threads, row, inner0);
+          if (p.view.nw)
+            Forward<N, T>::template load<kTiles>(p, g, smem.data(), tid, g.threads, row, inner0);
+          else
+            Forward<N, T>::load(p, g, smem.data(), tid, g.threads, row, inner0);
         for (int tid = 0; tid < g.threads; ++tid)
-          Forward<N, T>::template row_fetch<kTiles>(p, g, smem.data(), tid, row, inner0, regs[tid]);
+          if (p.view.nw)
+            Forward<N, T>::template row_fetch<kTiles>(p, g, smem.data(), tid, row, inner0, regs[tid]);
+          else
+            Forward<N, T>::row_fetch(p, g, smem.data(), tid, row, inner0, regs[tid]);
         std::memset(smem.data(), 0xFF, smem.size());  // aliasing: the row buffer is dead now
         for (int tid = 0; tid < g.threads; ++tid)
           Forward<N, T>::row_pass(g, smem.data(), tid, regs[tid]);
@@ -99,20 +107,22 @@ void run_inverse(const FftParams& p, int oh, int ow) {
             CoopInverse<N, T>::template col_step1<false>(p, g, smem.data(), tid, nth, row, inner0);
         for (int tid = 0; tid < nth; ++tid) CoopInverse<N, T>::col_step2(g, smem.data(), tid, nth);
         using I = CoopInverse<N, T>;
-        constexpr int N1 = I::N1, kTask = I::L::TASK_LINES;
+        constexpr int N1 = I::N1;
+        const bool half = I::L::half_tasks(g, nth);
+        const int task = half ? I::L::TASK_LINES / 2 : I::L::TASK_LINES, in_step1 = half ? 32 : 64;
         struct Item {
           float2 v[N1];
           bool on;
         };
-        for (int line0 = 0; line0 < g.lines1; line0 += kTask) {  // a warp's task: 32 lanes, two items each
-          std::vector<Item> items(64);
-          for (int i = 0; i < 64; ++i) items[i].on = I::row_step1_fft(p, g, smem.data(), line0, i, items[i].v);
-          for (int i = 0; i < 64; ++i) {
+        for (int line0 = 0; line0 < g.lines1; line0 += task) {  // a warp's task: 32 lanes, one or two items each
+          std::vector<Item> items(in_step1);
+          for (int i = 0; i < in_step1; ++i) items[i].on = I::row_step1_fft(p, g, smem.data(), line0, i, items[i].v);
+          for (int i = 0; i < in_step1; ++i) {
             float2 tw[N1];
             I::row_twiddles(i & 31, tw);
             if (items[i].on) I::row_step1_store(p, g, smem.data(), line0, i, items[i].v, tw);
           }
-          for (int i = 0; i < kTask * N1; ++i) I::row_step2(p, g, smem.data(), row, inner0, line0, i);
+          for (int i = 0; i < task * N1; ++i) I::row_step2(p, g, smem.data(), row, inner0, line0, i);
         }
       } else {
         for (int tid = 0; tid < g.threads; ++tid)
@@ -128,9 +138,15 @@ void run_inverse(const FftParams& p, int oh, int ow) {
           Inverse<N, T>::row_fetch(g, smem.data(), tid, regs[tid]);
         std::memset(smem.data() + g.off_b, 0xFF, smem.size() - g.off_b);  // mid is dead now
         for (int tid = 0; tid < g.threads; ++tid)
-          Inverse<N, T>::template row_pass<kTiles>(p, g, smem.data(), tid, row, inner0, regs[tid]);
+          if (p.view.nw)
+            Inverse<N, T>::template row_pass<kTiles>(p, g, smem.data(), tid, row, inner0, regs[tid]);
+          else
+            Inverse<N, T>::row_pass(p, g, smem.data(), tid, row, inner0, regs[tid]);
         for (int tid = 0; tid < g.threads; ++tid)
-          Inverse<N, T>::template store<kTiles>(p, g, smem.data(), tid, g.threads, row, inner0);
+          if (p.view.nw)
+            Inverse<N, T>::template store<kTiles>(p, g, smem.data(), tid, g.threads, row, inner0);
+          else
+            Inverse<N, T>::store(p, g, smem.data(), tid, g.threads, row, inner0);
       }
     }
   }

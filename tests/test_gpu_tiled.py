@@ -78,3 +78,36 @@ def test_untiled_module_refuses_what_the_tiled_one_takes():
     m = SpatialConvolutionFBFFT(1, 1, 3, 3)
     with pytest.raises(Exception):
         m.updateOutput(torch.zeros(1, 1, 150, 150, device="cuda"))
+
+
+# tiles above 32 pixels (cut, assembled and overlap-added by kernels of their own), spectra reused between the passes
+# of two steps (gradInput overlap-added), tiles of the output that end before the input does
+ROUTES = [
+    (oracle.Shape(2, 6, 4, 150, 141, 5, 4, 2, 1), 64, 64, "none"),
+    (oracle.Shape(1, 3, 2, 150, 100, 3, 3, 0, 0), 48, 64, "all"),   # plane-major inside
+    (oracle.Shape(1, 5, 3, 180, 150, 7, 7, 3, 3), 128, 128, "none"),
+    (oracle.Shape(1, 2, 3, 140, 260, 3, 5, 1, 0), 100, 128, "all"),
+    (oracle.Shape(2, 3, 4, 70, 61, 5, 4, 2, 1), 16, 16, "all"),
+    (oracle.Shape(2, 8, 16, 72, 60, 3, 3, 0, 0), 32, 32, "all"),
+    (oracle.Shape(1, 4, 3, 33, 40, 3, 3, 1, 1), 8, 8, "input"),
+    (oracle.Shape(2, 3, 5, 40, 40, 5, 5, 0, 0), 16, 16, "none"),    # 12-pixel output tiles: 3 cover 36 of the 40
+]
+
+
+@pytest.mark.parametrize("idx", range(len(ROUTES)))
+def test_routes_of_the_tiled_passes(idx):
+    s, th, tw, reuse = ROUTES[idx]
+    m = SpatialConvolutionFFTTiled(s.P, s.F, s.kW, s.kH, 1, 1, s.padW, s.padH, tw, th, reuse, accumulate=True)
+    gw = gb = 0.0
+    for step in range(2):  # other tensors in the second step, the gradients add up
+        x, w, go, b = _data(s, 400 + 10 * idx + step)
+        m.weight.copy_(torch.from_numpy(w))
+        m.bias.copy_(torch.from_numpy(b))
+        dx, dgo = torch.from_numpy(x).cuda(), torch.from_numpy(go).cuda()
+        out = m.updateOutput(dx).cpu().numpy()
+        gi = m.backward(dx, dgo, 0.6).cpu().numpy()
+        gw, gb = gw + oracle.acc_grad_weight(s, x, go, 0.6), gb + oracle.acc_grad_bias(s, go, 0.6)
+        assert _rel(out, oracle.update_output(s, x, w, b)) <= PASS_TOL
+        assert _rel(gi, oracle.update_grad_input(s, go, w)) <= PASS_TOL
+        assert _rel(m.gradWeight.cpu().numpy(), gw) <= PASS_TOL
+        assert _rel(m.gradBias.cpu().numpy(), gb) <= PASS_TOL

@@ -126,12 +126,7 @@ __device__ __forceinline__ void umma_tf32(uint32_t d_tmem, uint32_t a_tmem, uint
       ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
       : "memory");
 }
-// 8 or 16 columns of this warp's 32 lanes (a lane of the warp = a lane of tensor memory).
-__device__ __forceinline__ void tmem_store_cols(uint32_t taddr, const uint32_t (&r)[8]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-               ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-               : "memory");
-}
+// 16 columns of this warp's 32 lanes (a lane of the warp = a lane of tensor memory).
 __device__ __forceinline__ void tmem_store_cols(uint32_t taddr, const uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "

@@ -109,9 +109,9 @@ __device__ __forceinline__ void with_operand(const FftBatch<OPS>& b, int tile, B
   } else {
     if (tile < b.tile_end[0])
       body(b.p[0], b.g[0], tile, b.tiles_x[0]);
-    else if (tile < b.tile_end[1])
+    else if (OPS == 2 || tile < b.tile_end[1])
       body(b.p[1], b.g[1], tile - b.tile_end[0], b.tiles_x[1]);
-    else
+    else if constexpr (OPS > 2)
       body(b.p[2], b.g[2], tile - b.tile_end[1], b.tiles_x[2]);
   }
 }
@@ -344,13 +344,22 @@ long long coop_grid(const CoopShape& shape, long long tiles) {
   return shape.persistent && tiles > resident ? resident : tiles;
 }
 
-template <int N, int T, int OPS, bool PM>
-constexpr auto coop_kernel(bool inverse) {
-  constexpr CoopShape f = coop_shape(N, false, PM), i = coop_shape(N, true, PM);
-  static_assert(f.threads % 32 == 0 && i.threads % 32 == 0, "whole warps");
-  constexpr int blocks = f.blocks > i.blocks ? f.blocks : i.blocks;
-  static_assert(blocks * (N * CoopLayout<N, T>::PITCH2 * 8 + 1024) <= 228 * 1024, "shared memory of an SM");
-  return inverse ? fft2d_inverse_coop_kernel<N, T, OPS, PM> : fft2d_forward_coop_kernel<N, T, OPS, PM>;
+template <int N, int T, int OPS, bool INVERSE, bool PM>
+constexpr auto coop_kernel() {
+  constexpr CoopShape shape = coop_shape(N, INVERSE, PM);
+  static_assert(shape.threads % 32 == 0, "whole warps");
+  static_assert(shape.blocks * (N * CoopLayout<N, T>::PITCH2 * 8 + 1024) <= 228 * 1024, "shared memory of an SM");
+  if constexpr (INVERSE)
+    return fft2d_inverse_coop_kernel<N, T, OPS, PM>;
+  else
+    return fft2d_forward_coop_kernel<N, T, OPS, PM>;
+}
+template <int N, int T, int OPS, bool INVERSE, int MODE>
+constexpr auto line_kernel() {
+  if constexpr (INVERSE)
+    return fft2d_inverse_kernel<N, T, OPS, MODE>;
+  else
+    return fft2d_forward_kernel<N, T, OPS, MODE>;
 }
 
 // The kernels address the spectrum with 32-bit element offsets.
@@ -359,8 +368,8 @@ bool spectrum_fits(const FftParams& p, int N) {
   return bins * p.n_rows * p.kc < (1LL << 31);
 }
 
-template <int N, int OPS>
-cudaError_t run_batch(bool inverse, const FftParams* ops, int count, const RowSum* sum, cudaStream_t stream) {
+template <int N, int OPS, bool INVERSE>
+cudaError_t run_batch(const FftParams* ops, int count, const RowSum* sum, cudaStream_t stream) {
   constexpr int T = fft_tile(N);
   FftBatch<OPS> b{};
   long long tiles = 0;
@@ -373,9 +382,9 @@ cudaError_t run_batch(bool inverse, const FftParams* ops, int count, const RowSu
       b.p[i] = ops[i];
       if (ops[i].view.nw) mode = kTiles;
       if (ops[i].reference) mode = kReference;
-      b.g[i] = inverse ? inverse_geom(N, T, ops[i].h, ops[i].w, plane_major)
+      b.g[i] = INVERSE ? inverse_geom(N, T, ops[i].h, ops[i].w, plane_major)
                        : forward_geom(N, T, ops[i].h, ops[i].w, ops[i].off_y, ops[i].off_x, plane_major);
-      b.tiles_x[i] = ((inverse ? ops[i].n_inner : ops[i].kc) + T - 1) / T;
+      b.tiles_x[i] = ((INVERSE ? ops[i].n_inner : ops[i].kc) + T - 1) / T;
       tiles += (long long)b.tiles_x[i] * ops[i].n_rows;
       if (b.g[i].smem_bytes > smem) smem = b.g[i].smem_bytes;
     }
@@ -390,19 +399,18 @@ cudaError_t run_batch(bool inverse, const FftParams* ops, int count, const RowSu
   void (*kernel)(FftBatch<OPS>);
   long long blocks = tiles;
   if constexpr (N > 32) {
-    kernel = plane_major ? coop_kernel<N, T, OPS, true>(inverse) : coop_kernel<N, T, OPS, false>(inverse);
-    blocks = coop_grid(coop_shape(N, inverse, plane_major), tiles);
+    kernel = plane_major ? coop_kernel<N, T, OPS, INVERSE, true>() : coop_kernel<N, T, OPS, INVERSE, false>();
+    blocks = coop_grid(coop_shape(N, INVERSE, plane_major), tiles);
   } else {
     if (threads != block_threads<N, T>()) return cudaErrorInvalidConfiguration;
-    kernel = inverse ? fft2d_inverse_kernel<N, T, OPS, kPlanes> : fft2d_forward_kernel<N, T, OPS, kPlanes>;
-    if constexpr (N >= 8)
-      if (mode == kTiles)
-        kernel = inverse ? fft2d_inverse_kernel<N, T, OPS, kTiles> : fft2d_forward_kernel<N, T, OPS, kTiles>;
-    if constexpr (N >= 8 && OPS == 1)
-      if (mode == kReference)
-        kernel = inverse ? fft2d_inverse_kernel<N, T, 1, kReference> : fft2d_forward_kernel<N, T, 1, kReference>;
+    kernel = line_kernel<N, T, OPS, INVERSE, kPlanes>();
+    if constexpr (fft_modes_supported(N) && (OPS == 1 || !INVERSE))
+      if (mode == kTiles) kernel = line_kernel<N, T, OPS, INVERSE, kTiles>();
+    if constexpr (fft_modes_supported(N) && OPS == 1)
+      if (mode == kReference) kernel = line_kernel<N, T, OPS, INVERSE, kReference>();
   }
   if (mode != kPlanes && !fft_modes_supported(N)) return cudaErrorInvalidConfiguration;
+  if (mode == kTiles && INVERSE && OPS > 1) return cudaErrorInvalidConfiguration;  // no pass inverts two views at once
   if (mode == kReference && (OPS > 1 || ops[0].n_rows != 1 || ops[0].view.nw)) return cudaErrorInvalidConfiguration;
   cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
   if (e != cudaSuccess) return e;
@@ -411,24 +419,29 @@ cudaError_t run_batch(bool inverse, const FftParams* ops, int count, const RowSu
   return e;
 }
 
-template <int N>
-cudaError_t run_ops(bool inverse, const FftParams* ops, int count, const RowSum* sum, cudaStream_t s) {
-  if (count == 1) return run_batch<N, 1>(inverse, ops, count, sum, s);
-  return run_batch<N, kMaxFftOps>(inverse, ops, count, sum, s);
+// Sizes below 8 points are those of stand-alone transforms, one operand each.
+template <int N, bool INVERSE>
+cudaError_t run_ops(const FftParams* ops, int count, const RowSum* sum, cudaStream_t s) {
+  if (count == 1) return run_batch<N, 1, INVERSE>(ops, count, sum, s);
+  if constexpr (N >= 8)
+    return run_batch<N, INVERSE ? kMaxInverseOps : kMaxFftOps, INVERSE>(ops, count, sum, s);
+  else
+    return cudaErrorInvalidValue;
 }
 
-cudaError_t dispatch(bool inverse, const FftParams* ops, int count, const RowSum* sum, int N, cudaStream_t s) {
-  if (count < 1 || count > kMaxFftOps) return cudaErrorInvalidValue;
+template <bool INVERSE>
+cudaError_t dispatch(const FftParams* ops, int count, const RowSum* sum, int N, cudaStream_t s) {
+  if (count < 1 || count > (INVERSE ? kMaxInverseOps : kMaxFftOps)) return cudaErrorInvalidValue;
   for (int i = 0; i < count; ++i)
     if (ops[i].n_rows > 65535 || !spectrum_fits(ops[i], N)) return cudaErrorInvalidConfiguration;
   switch (N) {
-    case 2: return run_ops<2>(inverse, ops, count, sum, s);
-    case 4: return run_ops<4>(inverse, ops, count, sum, s);
-    case 8: return run_ops<8>(inverse, ops, count, sum, s);
-    case 16: return run_ops<16>(inverse, ops, count, sum, s);
-    case 32: return run_ops<32>(inverse, ops, count, sum, s);
-    case 64: return run_ops<64>(inverse, ops, count, sum, s);
-    case 128: return run_ops<128>(inverse, ops, count, sum, s);
+    case 2: return run_ops<2, INVERSE>(ops, count, sum, s);
+    case 4: return run_ops<4, INVERSE>(ops, count, sum, s);
+    case 8: return run_ops<8, INVERSE>(ops, count, sum, s);
+    case 16: return run_ops<16, INVERSE>(ops, count, sum, s);
+    case 32: return run_ops<32, INVERSE>(ops, count, sum, s);
+    case 64: return run_ops<64, INVERSE>(ops, count, sum, s);
+    case 128: return run_ops<128, INVERSE>(ops, count, sum, s);
   }
   return cudaErrorInvalidValue;
 }
@@ -454,11 +467,11 @@ void count_launch(int n) { g_launches.fetch_add(static_cast<uint64_t>(n), std::m
 uint64_t launch_count() { return g_launches.load(std::memory_order_relaxed); }
 
 cudaError_t launch_forward(const FftParams* ops, int count, int N, cudaStream_t stream) {
-  return dispatch(false, ops, count, nullptr, N, stream);
+  return dispatch<false>(ops, count, nullptr, N, stream);
 }
 
 cudaError_t launch_inverse(const FftParams* ops, int count, const RowSum* sum, int N, cudaStream_t stream) {
-  return dispatch(true, ops, count, sum, N, stream);
+  return dispatch<true>(ops, count, sum, N, stream);
 }
 
 namespace {

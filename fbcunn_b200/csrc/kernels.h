@@ -64,11 +64,12 @@ struct RowSum {
   int accumulate;
 };
 
-constexpr int kMaxFftOps = 3;
+constexpr int kMaxFftOps = 3;      // a backward call's operands
+constexpr int kMaxInverseOps = 2;  // and its products
 // Transform sizes whose kernels take tiles of images as planes (FftParams::view) and the reference's frequency
 // tensor as spectrum (FftParams::reference).
 constexpr bool fft_modes_supported(int N) { return N >= 8 && N <= 32; }
-// Transforms of up to kMaxFftOps operands in one launch (all of the same size N).
+// Transforms of several operands in one launch (all of the same size N).
 cudaError_t launch_forward(const FftParams* ops, int count, int N, cudaStream_t stream);
 cudaError_t launch_inverse(const FftParams* ops, int count, const RowSum* sum, int N, cudaStream_t stream);
 // batched 1-D real <-> half-complex transforms of contiguous rows (the row phases of the 2-D kernels)

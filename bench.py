@@ -3,14 +3,15 @@
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--layer C2] [--impl ours|reference]
 
-A step is the three nn passes (updateOutput, updateGradInput, accGradParameters) of one
-layer over one seeded synthetic batch; `value` is direct-convolution-equivalent TFLOP/s
+A step is the three nn passes of one layer, forward (updateOutput) and backward
+(updateGradInput and accGradParameters), over one seeded synthetic batch; `value` is direct-convolution-equivalent TFLOP/s
 (3 * 2*B*P*F*kH*kW*oH*oW flops per step) with the operands resident in HBM.  With N > 1
 ranks the global batch of 128 is split across ranks (strong scaling) and the weight
 gradient's spectrum is all-reduced inside accGradParameters.  `e2e` is the same step
 through the host-buffer entry points of the C ABI (pinned host memory, copies timed).
 The last stdout line is the short result object; the per-kernel and per-layer tables go
-to --detail-file.  Outside the timed region every timed layer is checked on sampled
+to --detail-file.  Per-kernel times come from steps of their own, outside the timed region:
+while kernels are timed one by one, those that otherwise share a launch run apart.  Outside the timed region every timed layer is checked on sampled
 planes against the fp64 direct convolution (`parity_checked`).
 `--impl reference` times the reference's own CPU convolution (compiled from its source
 under oracle/_ref) on a bounded batch slice with every host thread.
@@ -289,9 +290,8 @@ class LayerRun:
             self.m.attachCommunicator(*comm)
 
     def step(self):
-        self.m.updateOutput(self.x)
-        self.m.updateGradInput(self.x, self.go)
-        self.m.accGradParameters(self.x, self.go, 1.0)
+        self.m.forward(self.x)
+        self.m.backward(self.x, self.go, 1.0)
 
     def run_pass(self, i):
         if i == 0:
@@ -306,9 +306,8 @@ class LayerRun:
 
 
 def step_times(torch, capi, lib, run, iters):
-    """ms per step of three passes launched back to back (no flush, no profiling events), and the
-    same step replayed from a CUDA graph: what launch gaps cost on the small layers."""
-    capi.check(lib.fbfftconv_profile_enable(run.handle(), 0))
+    """ms per step launched back to back (no flush), and the same step replayed from a CUDA graph: what
+    launch gaps cost on the small layers."""
     out = {}
 
     def timed(fn):
@@ -343,22 +342,32 @@ def read_profile(handle):
             ms, n = ctypes.c_double(), ctypes.c_int()
             capi.check(capi.lib().fbfftconv_profile_read(handle, pi, si, ctypes.byref(ms), ctypes.byref(n)))
             if n.value:
-                out[(pi, sname)] = (ms.value, n.value, int(capi.lib().fbfftconv_profile_overlapped(handle, pi, si)) == 1)
+                out[(pi, sname)] = (ms.value, n.value)
+    return out
+
+
+def profile_steps(run, steps):
+    """Per-kernel times of `steps` steps whose kernels run one by one."""
+    from fbcunn_b200 import capi
+    lib = capi.lib()
+    capi.check(lib.fbfftconv_profile_enable(run.handle(), 1))
+    capi.check(lib.fbfftconv_profile_reset(run.handle()))
+    for _ in range(steps):
+        for i in range(3):
+            run.run_pass(i)
+    run.torch.cuda.synchronize()
+    out = read_profile(run.handle())
+    capi.check(lib.fbfftconv_profile_enable(run.handle(), 0))
     return out
 
 
 def kernel_table(L, B, prof, pk):
     rows = []
-    for (pi, sname), (ms, n, overlapped) in sorted(prof.items()):
+    for (pi, sname), (ms, n) in sorted(prof.items()):
         by, fl = stage_algorithmic(L, B, pi, sname)
         avg_s = ms / n / 1e3
         row = {"pass": PASSES[pi], "kernel": sname, "launches": n, "avg_us": 1e6 * avg_s, "total_ms": ms,
                "gbs": by / avg_s / 1e9 if avg_s > 0 else None}
-        if overlapped:
-            # ran next to the pass's other forward transform on the library's second stream: the time
-            # is wall time shared with that kernel, not this kernel's cost, so no rate is derived from it
-            row["overlapped"] = True
-            row["gbs"] = None
         if row["gbs"] is not None:
             row["frac_hbm"] = row["gbs"] / pk["hbm_gbs"]
         if fl:
@@ -449,8 +458,6 @@ def run_gpu_arm(args):
 
     # ---- timed region: K steps, device time, max over ranks --------------------
     lib = capi.lib()
-    capi.check(lib.fbfftconv_profile_enable(run.handle(), 1))
-    capi.check(lib.fbfftconv_profile_reset(run.handle()))
     launches0 = capi.kernel_launches()
     ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     barrier()
@@ -461,8 +468,9 @@ def run_gpu_arm(args):
     barrier()
     elapsed_ms = max_over_ranks(ev0.elapsed_time(ev1))
     launches = capi.kernel_launches() - launches0
-    prof = read_profile(run.handle())
-    capi.check(lib.fbfftconv_profile_enable(run.handle(), 0))
+    profiled_steps = min(args.steps, 10)
+    prof = profile_steps(run, profiled_steps)
+    barrier()
     device_status = int(lib.fbfftconv_tensor_core_status(0))
     if device_status != 0:
         raise SystemExit(f"tensor-core contraction reported device status {device_status}")
@@ -474,8 +482,7 @@ def run_gpu_arm(args):
         raise SystemExit(f"a bounded wait of the peer exchange gave up: status {run.m.peerExchangeStatus()}")
 
     kernels = kernel_table(L, local_b, prof, pk)
-    top = max((k for k in kernels if k["kernel"] != "allreduce" and not k.get("overlapped")),
-              key=lambda k: k["total_ms"])
+    top = max((k for k in kernels if k["kernel"] != "allreduce"), key=lambda k: k["total_ms"])
     by, fl = stage_algorithmic(L, local_b, PASSES.index(top["pass"]), top["kernel"])
     secs = top["avg_us"] / 1e6
     # the contraction is held against the tensor roofline where its intensity is above the
@@ -494,7 +501,7 @@ def run_gpu_arm(args):
                     "frac": achieved / pk["hbm_gbs"], "traffic": None, "algorithmic_bytes_per_launch": by}
     roofline["traffic"] = captured_traffic(name, top, L, local_b)
     roofline["avg_launch_us"] = top["avg_us"]
-    roofline["share_of_step"] = top["total_ms"] / elapsed_ms
+    roofline["share_of_step"] = top["total_ms"] / profiled_steps / ms_per_step
 
     # ---- e2e: host buffers through the *_host entry points ----------------------
     e2e = measure_e2e(torch, lib, run, L, local_b, world, barrier, max_over_ranks,
@@ -522,25 +529,26 @@ def run_gpu_arm(args):
             r = LayerRun(torch, lname, LL, lb, rank, comm, args.allreduce)
             for _ in range(3):
                 r.step()
-            capi.check(lib.fbfftconv_profile_enable(r.handle(), 1))
-            capi.check(lib.fbfftconv_profile_reset(r.handle()))
-            per_pass = []
-            for pi in range(3):
+
+            def cold(fn):
                 ts = []
                 for _ in range(args.layer_iters):
                     flush.zero_()
                     a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
                     barrier()
                     a.record()
-                    r.run_pass(pi)
+                    fn()
                     b.record()
                     barrier()
                     ts.append(max_over_ranks(a.elapsed_time(b)))
-                ms = statistics.median(ts)
+                return statistics.median(ts)
+
+            per_pass = []
+            for pi in range(3):
+                ms = cold(lambda: r.run_pass(pi))
                 per_pass.append({"pass": PASSES[pi], "ms": ms, "tflops": conv_flops(LL) / (ms / 1e3) / 1e12})
-            prof_l = read_profile(r.handle())
-            layers[lname] = {"fft_size": fft_size(LL), "local_batch": lb, "passes": per_pass,
-                             "kernels": kernel_table(LL, lb, prof_l, pk)}
+            layers[lname] = {"fft_size": fft_size(LL), "local_batch": lb, "passes": per_pass, "cold_step_ms": cold(r.step),
+                             "kernels": kernel_table(LL, lb, profile_steps(r, args.layer_iters), pk)}
             if world == 1:
                 layers[lname]["step_ms"] = step_times(torch, capi, lib, r, args.layer_iters)
             if parity is not None and lname != name:
@@ -579,8 +587,8 @@ def run_gpu_arm(args):
                 json.dump(detail, f, indent=1)
         except OSError as e:
             sys.stderr.write(f"bench detail not written: {e}\n")
-        # per layer: sum of the three per-pass medians (ms), each timed after an L2 flush
-        layers_step_ms = {k: sig(sum(p["ms"] for p in v["passes"])) for k, v in layers.items()}
+        # per layer: median step (ms), each timed after an L2 flush
+        layers_step_ms = {k: sig(v["cold_step_ms"]) for k, v in layers.items()}
         line = {
             "metric": METRIC, "value": sig(value, 5), "unit": "TFLOP/s", "n_gpus": world, "steps": args.steps,
             "warmup": max(args.warmup, 3), "ms_per_step": sig(ms_per_step, 5), "higher_is_better": True,

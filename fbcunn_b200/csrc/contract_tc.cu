@@ -126,6 +126,16 @@ __device__ __forceinline__ void umma_tf32(uint32_t d_tmem, uint32_t a_tmem, uint
       ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
       : "memory");
 }
+// Both operands in shared memory.
+__device__ __forceinline__ void umma_tf32(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                          uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
+      : "memory");
+}
 // 16 columns of this warp's 32 lanes (a lane of the warp = a lane of tensor memory).
 __device__ __forceinline__ void tmem_store_cols(uint32_t taddr, const uint32_t (&r)[16]) {
   asm volatile(
@@ -301,10 +311,10 @@ struct MapCache {
 };
 MapCache g_maps;
 
-template <int WBNC, bool A_MN, bool B_MN>
+template <int WBNC, bool A_TMEM, bool A_MN, bool B_MN>
 cudaError_t launch_wide_as(const ContractParams& p, cudaStream_t stream) {
   using namespace wide;
-  using TL = WideTile<WBNC>;
+  using TL = WideTile<WBNC, A_TMEM>;
   CUtensorMap map_a, map_b;
   if (!g_maps.get(operand_key(p.a, p.m, p.k, p.lda, p.bins, WBM, TL::KB, p.a_mn != 0, true), &map_a) ||
       !g_maps.get(operand_key(p.b, p.n, p.k, p.ldb, p.bins, WBNC, TL::KB, p.b_mn != 0, false), &map_b))
@@ -326,32 +336,41 @@ cudaError_t launch_wide_as(const ContractParams& p, cudaStream_t stream) {
   t.s_b1_im = -sa * sb;
   t.s_b2_re = sb;
   t.s_b2_im = sa;
-  cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(contract_tc_wide_kernel<WBNC, A_MN, B_MN>), TL::SMEM_BYTES);
+  const auto kernel = contract_tc_wide_kernel<WBNC, A_TMEM, A_MN, B_MN>;
+  cudaError_t e = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), TL::SMEM_BYTES);
   if (e != cudaSuccess) return e;
   const int sms = sm_count();
   const int grid = (int)(total < sms ? total : sms);
-  e = launch_dependent(contract_tc_wide_kernel<WBNC, A_MN, B_MN>, dim3(grid), W_THREADS, TL::SMEM_BYTES, stream, map_a,
-                       map_b, t);
+  e = launch_dependent(kernel, dim3(grid), W_THREADS, TL::SMEM_BYTES, stream, map_a, map_b, t);
   count_launch();
   return e;
 }
 
-template <int WBNC>
+template <int WBNC, bool A_TMEM>
 cudaError_t launch_wide(const ContractParams& p, cudaStream_t stream) {
-  if (p.a_mn) return p.b_mn ? launch_wide_as<WBNC, true, true>(p, stream) : launch_wide_as<WBNC, true, false>(p, stream);
-  return p.b_mn ? launch_wide_as<WBNC, false, true>(p, stream) : launch_wide_as<WBNC, false, false>(p, stream);
+  if (p.a_mn)
+    return p.b_mn ? launch_wide_as<WBNC, A_TMEM, true, true>(p, stream)
+                  : launch_wide_as<WBNC, A_TMEM, true, false>(p, stream);
+  return p.b_mn ? launch_wide_as<WBNC, A_TMEM, false, true>(p, stream)
+                : launch_wide_as<WBNC, A_TMEM, false, false>(p, stream);
 }
 
 }  // namespace
 
 // The tile's column count follows the problem's: the smallest of 16 / 32 / 64 / 128 complex columns
-// that covers it, 128 beyond.
+// that covers it, 128 beyond.  At 128 columns A goes through shared memory up to a depth of 80 (kShortDepth), which
+// leaves tensor memory for two accumulators: such tiles are bound by the draining of one.  us per call, A in tensor
+// memory / in shared memory, bins x rows x columns: 2112 x 128 x 128 at depth 16 81 / 72, 64 127 / 111, 70 144 / 135,
+// 96 174 / 183, 128 209 / 228; 544 x 300 x 200 at 32 127 / 110, 64 176 / 154, 70 186 / 174, 96 217 / 220,
+// 384 620 / 741.
 cudaError_t launch_contract_tc(const ContractParams& p, cudaStream_t stream) {
   if (!contract_tc_supported(p)) return cudaErrorInvalidValue;
-  if (p.ldc <= 16) return launch_wide<16>(p, stream);
-  if (p.ldc <= 32) return launch_wide<32>(p, stream);
-  if (p.ldc <= 64) return launch_wide<64>(p, stream);
-  return launch_wide<128>(p, stream);
+  if (p.ldc <= 16) return launch_wide<16, true>(p, stream);
+  if (p.ldc <= 32) return launch_wide<32, true>(p, stream);
+  if (p.ldc <= 64) return launch_wide<64, true>(p, stream);
+  constexpr int kShortDepth = 80;
+  if (p.k <= kShortDepth) return launch_wide<128, false>(p, stream);
+  return launch_wide<128, true>(p, stream);
 }
 
 // Runs wait_probe_kernel and returns 1 when the wait gave up as designed, 0 when it did not,

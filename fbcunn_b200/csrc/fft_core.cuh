@@ -239,7 +239,7 @@ static inline bool cooperative(int N) { return N > 32; }
 // blocks share an SM's memory.
 constexpr int fft_tile(int N) { return N > 64 ? 1 : N > 32 ? 4 : N > 16 ? 8 : 16; }
 // Threads of a cooperative block, blocks per SM, and whether the blocks are persistent or one per tile.  With the
-// column buffer alone in shared memory (69 KB at 128 points, 74 at 64) two or three blocks fit an SM; what bounds
+// column buffer alone in shared memory (70 KB at 128 points, 76 at 64) two or three blocks fit an SM; what bounds
 // the plane-major kernels is instruction issue and the latency of a thread's own chain, and a shape below 128
 // registers a thread spills.  Bin-major spectra are bound by their 8- and 32-byte pieces: the blocks that share a
 // sector (neighbouring tiles) have to meet it while it is in L2.  Persistent blocks drift apart without bound,

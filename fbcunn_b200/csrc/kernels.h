@@ -22,9 +22,9 @@ int sm_count();
 cudaError_t ensure_dynamic_smem(const void* kernel, int bytes);
 
 // ---- programmatic dependent launch -----------------------------------------------------------
-// Every kernel of a pass is launched so that its blocks may be placed, SM by SM, as the blocks of the kernel
-// before it leave, instead of after the last of them has gone: they do what needs no input and wait in
-// grid_dependency_wait() until that kernel has finished and its writes are visible.  Such a kernel calls
+// Every kernel of a pass is launched so that it is set up while the kernel before it runs and its blocks start as
+// soon as the last block of that one has exited, without waiting for the flush of its writes first: they do what
+// needs no input and wait in grid_dependency_wait() until that kernel has finished and its writes are visible.  Such a kernel calls
 // grid_dependency_wait() in every block before its first access to global memory (also when it only writes:
 // an earlier kernel may still be reading the buffer), which makes the order transitive along the stream.
 // No kernel here triggers its successor early (griddepcontrol.launch_dependents): successors placed beside

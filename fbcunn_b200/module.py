@@ -40,12 +40,6 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
     return t.data_ptr() if t is not None else None
 
 
-def _share_memory(a: torch.Tensor, b: torch.Tensor) -> bool:
-    """Whether two contiguous tensors overlap."""
-    return (a.data_ptr() < b.data_ptr() + b.numel() * b.element_size()
-            and b.data_ptr() < a.data_ptr() + a.numel() * a.element_size())
-
-
 def _device_index(device: torch.device) -> int:
     return device.index if device.index is not None else torch.cuda.current_device()
 
@@ -61,12 +55,6 @@ def _stream(device) -> int:
 
 def _is_number(x) -> bool:
     return isinstance(x, (int, float)) and not isinstance(x, bool)
-
-
-def own_passes(module, passes) -> bool:
-    """Whether `module` runs the two given functions as its backward passes, so that one call may stand for both."""
-    return (getattr(module.updateGradInput, "__func__", None) is passes[0]
-            and getattr(module.accGradParameters, "__func__", None) is passes[1])
 
 
 class SpatialConvolutionFBFFT:
@@ -204,7 +192,9 @@ class SpatialConvolutionFBFFT:
         """updateGradInput and accGradParameters (fbcunn/SpatialConvolutionFFT.lua:405-416) in one native
         call, which transforms gradOutput once for both.  Passes that a subclass, the object itself or a
         patched class brings are called one after the other."""
-        if not own_passes(self, _PASSES):
+        cls, own = type(self), self.__dict__
+        if (cls.updateGradInput is not _GRAD_INPUT or cls.accGradParameters is not _GRAD_PARAMETERS
+                or "updateGradInput" in own or "accGradParameters" in own):
             self.updateGradInput(input, gradOutput)
             self.accGradParameters(input, gradOutput, scale)
             return self.gradInput
@@ -217,8 +207,8 @@ class SpatialConvolutionFBFFT:
             self.gradInput = torch.empty_like(input)
         capi.check(capi.lib().fbfftconv_backward(
             h, input.data_ptr(), gradOutput.data_ptr(), self.weight.data_ptr(), self.gradInput.data_ptr(),
-            self.gradWeight.data_ptr(), _ptr(self.gradBias), 1.0 if scale is None else float(scale),
-            _stream(self.device)))
+            self.gradWeight.data_ptr(), None if self.gradBias is None else self.gradBias.data_ptr(),
+            1.0 if scale is None else float(scale), _stream(self.device)))
         return self.gradInput
 
     def zeroGradParameters(self):
@@ -337,7 +327,7 @@ class SpatialConvolutionFBFFT:
 
 
 # the backward passes as they are defined above, whatever becomes of the class attributes
-_PASSES = (SpatialConvolutionFBFFT.updateGradInput, SpatialConvolutionFBFFT.accGradParameters)
+_GRAD_INPUT, _GRAD_PARAMETERS = SpatialConvolutionFBFFT.updateGradInput, SpatialConvolutionFBFFT.accGradParameters
 
 
 class SpatialConvolutionFBFFTGemm(SpatialConvolutionFBFFT):
@@ -446,25 +436,24 @@ class FFTWrapper:
         assert frequency.shape[-3] == n_fft // 2 + 1
         h, w = time.shape[-2:]
         planes = time.numel() // (h * w)
-        scratch = self._scratch(planes, n_fft, time, frequency)
+        t, f = time.data_ptr(), frequency.data_ptr()
         capi.check(capi.lib().fbfftconv_fft2d_reference_layout(
-            _ptr(time), _ptr(frequency), _ptr(scratch), planes, h, w, n_fft, self.padUp, self.padLeft, stream))
+            t, f, self._scratch(planes, n_fft, time, t, f), planes, h, w, n_fft, self.padUp, self.padLeft, stream))
         return frequency
 
-    def _scratch(self, planes, n_fft, time, frequency):
-        """The block that the library goes through where it does not transform between the two tensors
-        directly: its own half spectrum of `planes` planes, which a kernel converts to / from the reference's
-        tensor, and for transforms in place.  Kept between calls of the same size.  Elsewhere the block is not
-        touched: `frequency` stands in for it."""
-        if self._half_along_rows(n_fft) and not _share_memory(time, frequency):
-            return frequency
-        device = time.device
+    def _scratch(self, planes, n_fft, time, t, f):
+        """Address of the block that the library goes through where it does not transform between the two tensors
+        (at t and f) directly: its own half spectrum of `planes` planes, which a kernel converts to / from the
+        reference's tensor, and for transforms in place.  Kept between calls of the same size.  Elsewhere the block
+        is not touched: the frequency tensor stands in for it."""
         need = (n_fft // 2 + 1) * n_fft * ((planes + 3) // 4 * 4) * 8  # fbfftconv_spectrum_bytes(n_fft, 1, planes)
+        if 8 <= n_fft <= 32 and (t >= f + need or f >= t + 4 * time.numel()):
+            return f
         buf = getattr(self, "_scratch_buf", None)
-        if buf is None or buf.numel() < need or buf.device != device:
-            buf = torch.empty(need, dtype=torch.uint8, device=device)
+        if buf is None or buf.numel() < need or buf.device != time.device:
+            buf = torch.empty(need, dtype=torch.uint8, device=time.device)
             self._scratch_buf = buf
-        return buf
+        return buf.data_ptr()
 
     def ffti_reference_layout(self, time: torch.Tensor, frequency: torch.Tensor, batchDims: int):
         assert 1 <= batchDims <= 2 and time.is_cuda and time.dtype == torch.float32 and time.is_contiguous()
@@ -480,7 +469,7 @@ class FFTWrapper:
         n_fft = frequency.shape[-2]
         h, w = time.shape[-2:]
         planes = time.numel() // (h * w)
-        scratch = self._scratch(planes, n_fft, time, frequency)
+        t, f = time.data_ptr(), frequency.data_ptr()
         capi.check(capi.lib().fbfftconv_ifft2d_reference_layout(
-            _ptr(frequency), _ptr(time), _ptr(scratch), planes, h, w, n_fft, self.padUp, self.padLeft, stream))
+            f, t, self._scratch(planes, n_fft, time, t, f), planes, h, w, n_fft, self.padUp, self.padLeft, stream))
         return time

@@ -20,7 +20,7 @@ from typing import Callable, List, Optional, Tuple
 import torch
 
 from . import capi
-from .module import SpatialConvolutionFBFFT, memoryReuseAll, memoryReuseNone, own_passes
+from .module import SpatialConvolutionFBFFT, memoryReuseAll, memoryReuseNone
 from .tiled import SpatialConvolutionFFTTiled
 
 Candidate = Tuple[str, Callable[[], SpatialConvolutionFBFFT]]
@@ -166,7 +166,9 @@ class SpatialConvolution:
         return self.updateOutput(input)
 
     def backward(self, input, gradOutput, scale=None):
-        if not own_passes(self, _PASSES):
+        cls, own = type(self), self.__dict__
+        if (cls.updateGradInput is not _GRAD_INPUT or cls.accGradParameters is not _GRAD_PARAMETERS
+                or "updateGradInput" in own or "accGradParameters" in own):
             self.updateGradInput(input, gradOutput)
             self.accGradParameters(input, gradOutput, scale)
             return self.gradInput
@@ -185,4 +187,4 @@ class SpatialConvolution:
 
 
 # the backward passes as they are defined above, whatever becomes of the class attributes
-_PASSES = (SpatialConvolution.updateGradInput, SpatialConvolution.accGradParameters)
+_GRAD_INPUT, _GRAD_PARAMETERS = SpatialConvolution.updateGradInput, SpatialConvolution.accGradParameters

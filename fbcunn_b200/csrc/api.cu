@@ -714,15 +714,18 @@ Operand grad_output_operand(const fbfftconv_handle* h, int stage, const float* g
 }
 
 // Whether a transform shares a launch with the pass's other ones.  Up to 32 points always: one wave fewer, and no
-// launch gap.  The cooperative kernels of the larger sizes only where it has too few tiles to fill the GPU (four
-// per SM): small transforms beside each other fill it better, while a large one loses in the kernel that looks its
-// operand up.  updateOutput / backward, us, sharing up to 0, 4 and 16 tiles per SM: 16 x 3 -> 96 planes of
-// 128 x 128 (11 x 11 filters) 118 / 166, 110 / 154, 110 / 151; 8 x 32 -> 64 of 64 x 64 (9 x 9) 63 / 130, 56 / 116,
-// 56 / 116; 32 x 16 -> 64 of 100 x 100 (7 x 7) 349 / 678, 341 / 678, 355 / 693.  (Every operand shared wherever one
-// is small: 4 x 64 -> 128 of 128 x 128 with 5 x 5 filters 1010 / 1756 against 796 / 1544.)
+// launch gap.  The cooperative kernels of the larger sizes only up to so many tiles per SM: a transform that keeps the
+// GPU busy by itself gains little beside others and loses in the kernel that looks its operand up, least of all at 64
+// points, most where that kernel spills (128 points, bin-major).  updateOutput / backward, us, sharing up to 0, 4, 8
+// and 24 tiles per SM: 64 points, 48 x 60 -> 60 planes 154 / 264, 154 / 264, 147 / 257, 148 / 257; 128 x 8 -> 32 96 /
+// 206, 90 / 206, 91 / 202, 91 / 202; 40 x 64 -> 200 332 / 607, 332 / 607, 332 / 607, 327 / 603.  128 points,
+// plane-major, 64 x 3 -> 16 planes 82 / 122, 76 / 122, 76 / 117, 76 / 117; 128 x 3 -> 16 148 / 199, 142 / 199, 142 /
+// 199, 142 / 195; bin-major, 16 x 16 -> 32 planes 158 / 313, 155 / 307, 155 / 308, 155 / 307 (up to 16); 128 x 8 -> 32
+// 473 / 967, 475 / 967, 484 / 967, 484 / 968.  (Every operand shared wherever one is small: 4 x 64 -> 128 planes of
+// 128 x 128 1010 / 1756 against 796 / 1544.)
 bool shares_launch(int N, const FftParams& p) {
-  const int T = fft_tile(N);
-  return N <= 32 || (long long)p.n_rows * ((p.n_inner + T - 1) / T) < 4LL * sm_count();
+  const int T = fft_tile(N), tiles_per_sm = N <= 64 ? 24 : p.spec_bin == 1 ? 16 : 4;
+  return N <= 32 || (long long)p.n_rows * ((p.n_inner + T - 1) / T) < (long long)tiles_per_sm * sm_count();
 }
 
 int forward_transforms(fbfftconv_handle* h, int pass, const Operand* ops, int count, cudaStream_t s) {

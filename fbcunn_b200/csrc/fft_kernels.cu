@@ -166,8 +166,7 @@ __device__ __forceinline__ void prefetch_l2(const void* p) {
   asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }
 
-// The cooperative kernels look the operand up per tile (only operands that do not fill the GPU by themselves reach
-// the merged form): `tile` becomes the tile's number inside the operand.
+// The cooperative kernels look the operand up per tile: `tile` becomes the tile's number inside the operand.
 template <int OPS>
 __device__ __forceinline__ int operand_of_tile(const FftBatch<OPS>& b, int& tile) {
   if constexpr (OPS == 1) {

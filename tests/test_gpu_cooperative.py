@@ -53,9 +53,9 @@ def test_forward_and_inverse(n, shape, plane_major):
     assert np.abs(back.cpu().numpy() - want).max() <= TOL * np.abs(want).max()
 
 
-# layers with one transform that fills the GPU (four tiles per SM) beside ones that do not: 64 points bin-major, 128
-# points plane-major, 128 points bin-major
-@pytest.mark.parametrize("s", [oracle.Shape(300, 8, 2, 40, 38, 3, 3), oracle.Shape(200, 3, 1, 70, 66, 3, 2, 1, 0),
+# Layers with one transform that keeps the GPU busy by itself beside small ones: beyond 24 tiles per SM at 64 points, 16
+# at 128 points plane-major, 4 bin-major.
+@pytest.mark.parametrize("s", [oracle.Shape(1800, 5, 1, 33, 34, 3, 3), oracle.Shape(810, 3, 1, 66, 65, 3, 2, 1, 0),
                                oracle.Shape(100, 6, 1, 66, 70, 2, 3)], ids=lambda s: "x".join(map(str, (s.B, s.P, s.iH))))
 def test_large_and_small_operands(s):
     def rel(a, ref):

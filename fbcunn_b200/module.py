@@ -105,7 +105,7 @@ class SpatialConvolutionFBFFT:
         assert exchange in ("auto", "nccl")
         self._exchange = exchange
         # no more scratch than the passes need (FBFFTCONV_MIN_WORKSPACE)
-        self._min_workspace = bool(min_workspace)
+        self._min_workspace = capi.MIN_WORKSPACE if min_workspace else 0
         shape_w = (self.nOutputPlane, self.nInputPlane, self.kH, self.kW)
         self.weight = torch.empty(shape_w, dtype=torch.float32, device=self.device)
         self.bias = torch.empty(self.nOutputPlane, dtype=torch.float32, device=self.device)
@@ -292,7 +292,7 @@ class SpatialConvolutionFBFFT:
                 (capi.BIN_MAJOR_ONLY if self._contraction == "bin_major" else 0) | \
                 (capi.ALLREDUCE_SPATIAL if self._allreduce == "spatial" else 0) | \
                 (capi.EXCHANGE_NCCL if self._exchange == "nccl" else 0) | \
-                (capi.MIN_WORKSPACE if self._min_workspace else 0) | \
+                self._min_workspace | \
                 (capi.REUSE_INPUT if memoryReuseInput in self.memoryReusePolicy else 0) | \
                 (capi.REUSE_OUTPUT if memoryReuseOutput in self.memoryReusePolicy else 0) | \
                 (capi.REUSE_WEIGHT if memoryReuseWeight in self.memoryReusePolicy else 0)
